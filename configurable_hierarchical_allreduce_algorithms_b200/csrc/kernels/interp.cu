@@ -22,11 +22,11 @@
 #include "../api/program_handle.h"
 #include "../symm/comm.h"
 #include "common.cuh"
+#include "span.cuh"
 
 namespace chb {
 
 constexpr int kInterpThreads = 512;
-constexpr int kMaxSrc = 40;              // sources per step (incl. the accumulate operand)
 constexpr long long kSmallStepElems = 16 << 10;  // steps below this many elements are run whole, by one CTA
 
 struct DevStep { long long dst_off; long long count; int dst_buf; int nsrc; int src_begin; unsigned flags; };
@@ -175,84 +175,30 @@ static std::vector<char> make_blob(const Program& p, long long* rank_table_bytes
 }
 
 // ------------------------------------------------------------------ one step (or one tile of it)
-// Elements [e0, e0 + cnt) of step `st`, strided over `nparts` CTAs of which this one is `part`.
-// Sources are combined left to right (the order in which the reference receives and reduces), but
-// their loads are issued kSrcGroup sources at a time and two vectors deep, so that every thread keeps
-// 128 bytes of NVLink round trips in flight whether a step has one remote source or P-1 of them.
-constexpr int kSrcGroup = 2;
-
-// 256-bit reduce loop over vectors [j0, nw) strided by TT: G sources x UW vectors in flight per thread.
-// (not inlined: each variant gets a register allocation of its own instead of inflating the interpreter's)
-template <typename T, int G, int UW>
-__device__ __noinline__ void reduce_loop32(const char* const* s_ptr, char* dst, int nsrc, long long j0, long long nw,
-                                              long long TT, int op, bool do_scale, float scale) {
-  using Acc = typename Elem<T>::Acc;
-  constexpr int VE = Elem<T>::kPerVec;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  for (; j0 < nw; j0 += TT * UW) {
-    Acc a[UW][2][VE];
-    for (int s = 0; s < nsrc; s += G) {
-      uint4 x[G][UW][2];
-#pragma unroll
-      for (int gi = 0; gi < G; ++gi) {
-        if (s + gi < nsrc) {
-          const char* p0 = s_ptr[s + gi];
-#pragma unroll
-          for (int u = 0; u < UW; ++u) {
-            const long long j = j0 + (long long)u * TT;
-            if (j < nw) ld32_cg(p0 + j * 32, x[gi][u][0], x[gi][u][1]);
-            else x[gi][u][0] = x[gi][u][1] = zero;
-          }
-        }
-      }
-#pragma unroll
-      for (int gi = 0; gi < G; ++gi) {
-        if (s + gi < nsrc) {
-          if (gi == 0 && s == 0) {
-#pragma unroll
-            for (int u = 0; u < UW; ++u) { vec_to_acc<T>(x[0][u][0], a[u][0]); vec_to_acc<T>(x[0][u][1], a[u][1]); }
-          } else {
-#pragma unroll
-            for (int u = 0; u < UW; ++u) { vec_combine<T>(op, x[gi][u][0], a[u][0]); vec_combine<T>(op, x[gi][u][1], a[u][1]); }
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < UW; ++u) {
-      const long long j = j0 + (long long)u * TT;
-      if (j < nw) {
-        if (do_scale) { acc_scale<T>(a[u][0], scale); acc_scale<T>(a[u][1], scale); }
-        st32(dst + j * 32, acc_to_vec<T>(a[u][0]), acc_to_vec<T>(a[u][1]));
-      }
-    }
-  }
-}
-
+// Elements [e0, e0 + cnt) of step `st`, by this CTA.  Sources are combined left to right (the order in which the
+// reference receives and reduces); the loops are in span.cuh.
 template <typename T>
-__device__ __forceinline__ void run_step(const DevStep& st, const DevSrc* __restrict__ srcs, const World& w,
+__device__ __forceinline__ bool set_step(const DevStep& st, const DevSrc* __restrict__ srcs, const World& w,
                                          const IoTable& io, int rank, long long e0, long long cnt,
-                                         unsigned part, unsigned nparts,
-                                         int op, float scale, const char** s_ptr, int* s_meta, const long long* limit) {
-  using Acc = typename Elem<T>::Acc;
-  constexpr int VE = Elem<T>::kPerVec;
-  constexpr int G = kSrcGroup;
+                                         int op, float scale, SpanArgs* a, const long long* limit) {
   const int tid = threadIdx.x;
-  const bool acc = (st.flags & 0x100u) != 0;
-  const int nsrc = st.nsrc + (acc ? 1 : 0);
-  __syncthreads();  // previous step's readers of s_ptr are done
-  if (tid < nsrc || tid == kMaxSrc) {
-    if (tid == kMaxSrc) {
-      char* base = st.dst_buf == 0 ? const_cast<char*>(io.in[rank]) : (st.dst_buf == 1 ? io.out[rank] : w.work[rank]);
-      s_ptr[kMaxSrc] = base + (st.dst_off + e0) * (long long)sizeof(T);
-    } else if (acc && tid == 0) {
-      char* base = st.dst_buf == 1 ? io.out[rank] : w.work[rank];
-      s_ptr[0] = base + (st.dst_off + e0) * (long long)sizeof(T);
-    } else {
-      const DevSrc s = srcs[st.src_begin + tid - (acc ? 1 : 0)];
-      const char* base = s.buf == 0 ? io.in[s.peer] : (s.buf == 1 ? io.out[s.peer] : w.work[s.peer]);
-      s_ptr[tid] = base + (s.off + e0) * (long long)sizeof(T);
-    }
+  const int acc = (st.flags & 0x100u) != 0 ? 1 : 0;
+  if (tid < st.nsrc) {
+    const DevSrc s = srcs[st.src_begin + tid];
+    const char* base = s.buf == 0 ? io.in[s.peer] : (s.buf == 1 ? io.out[s.peer] : w.work[s.peer]);
+    a->src[tid + acc] = base + (s.off + e0) * (long long)sizeof(T);
+  }
+  if (tid == 0) {
+    char* base = st.dst_buf == 0 ? const_cast<char*>(io.in[rank]) : (st.dst_buf == 1 ? io.out[rank] : w.work[rank]);
+    a->dst[0] = base + (st.dst_off + e0) * (long long)sizeof(T);
+    if (acc) a->src[0] = a->dst[0];
+    a->nsrc = st.nsrc + acc;
+    a->ndst = 1;
+    a->count = cnt;
+    a->op = op;
+    a->do_scale = (st.flags & OPF_FINAL) && scale != 1.0f;
+    a->plain = a->nsrc == 1 && !a->do_scale;
+    a->scale = scale;
   }
 #ifdef CHB_CHECK_BOUNDS
   // checked build: the same range test as on the host, on the values the kernel actually uses
@@ -262,98 +208,11 @@ __device__ __forceinline__ void run_step(const DevStep& st, const DevSrc* __rest
       const DevSrc s = srcs[st.src_begin + j];
       ok = ok && s.off >= 0 && s.off + st.count <= limit[s.buf] && s.peer >= 0 && s.peer < w.P;
     }
-    s_meta[0] = ok ? 0 : -1;
-    if (!ok) record_timeout(w.ctrl[rank], ST_OUT_OF_RANGE, rank, -1, -1, (unsigned long long)st.dst_off, (unsigned long long)st.count);
+    if (!ok) { a->nsrc = -1; record_timeout(w.ctrl[rank], ST_OUT_OF_RANGE, rank, -1, -1, (unsigned long long)st.dst_off, (unsigned long long)st.count); }
   }
-  __syncthreads();
-  if (s_meta[0] < 0) return;
 #endif
   __syncthreads();
-  // widest vector every pointer allows (every thread works it out from the shared table: no second barrier)
-  unsigned long long m = (unsigned long long)s_ptr[kMaxSrc];
-  for (int i = 0; i < nsrc; ++i) m |= (unsigned long long)s_ptr[i];
-  const int align_level = (m & 31ull) == 0ull ? 2 : ((m & 15ull) == 0ull ? 1 : 0);
-  const bool aligned = align_level != 0;
-  char* dst = const_cast<char*>(s_ptr[kMaxSrc]);
-  const bool do_scale = (st.flags & OPF_FINAL) && scale != 1.0f;
-  const long long count = cnt;
-  const long long nvec = aligned ? count / VE : 0;
-  const long long TT = (long long)nparts * blockDim.x;
-  const long long g = (long long)part * blockDim.x + tid;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  long long i0 = g;
-  if (align_level == 2) {
-    // 256-bit accesses on pairs of vectors; a last odd vector is left to the 128-bit loop
-    const long long nw = nvec / 2;
-    long long j0 = g;
-    if (nsrc == 1 && !do_scale) {
-      // plain copy (gather / broadcast steps, staging): no arithmetic, full tiles with twice the bytes in flight
-      constexpr int UC = 4;
-      const char* p = s_ptr[0] + j0 * 32;
-      char* d = dst + j0 * 32;
-      const long long stride = TT * 32;
-      for (; j0 + (long long)(UC - 1) * TT < nw; j0 += TT * UC) {
-        uint4 lo[UC], hi[UC];
-#pragma unroll
-        for (int u = 0; u < UC; ++u) ld32_cg(p + u * stride, lo[u], hi[u]);
-#pragma unroll
-        for (int u = 0; u < UC; ++u) st32(d + u * stride, lo[u], hi[u]);
-        p += UC * stride;
-        d += UC * stride;
-      }
-    }
-    // a tile with at most one vector per thread is bound by the depth of its chain of round trips: four sources at
-    // a time; longer tiles by bytes in flight: two sources, two vectors deep (the same 128 bytes per thread)
-    if (nw <= TT) reduce_loop32<T, 4, 1>(s_ptr, dst, nsrc, j0, nw, TT, op, do_scale, scale);
-    else reduce_loop32<T, kSrcGroup, 2>(s_ptr, dst, nsrc, j0, nw, TT, op, do_scale, scale);
-    i0 = nw * 2 + g;
-  }
-  constexpr int U = 2;
-  for (; i0 < nvec; i0 += TT * U) {
-    Acc a[U][VE];
-    for (int s = 0; s < nsrc; s += G) {
-      uint4 x[G][U];
-#pragma unroll
-      for (int gi = 0; gi < G; ++gi) {
-        if (s + gi < nsrc) {
-          const char* p0 = s_ptr[s + gi];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const long long i = i0 + (long long)u * TT;
-            x[gi][u] = (i < nvec) ? ld16_cg(p0 + i * 16) : zero;
-          }
-        }
-      }
-#pragma unroll
-      for (int gi = 0; gi < G; ++gi) {
-        if (s + gi < nsrc) {
-          if (gi == 0 && s == 0) {
-#pragma unroll
-            for (int u = 0; u < U; ++u) vec_to_acc<T>(x[0][u], a[u]);
-          } else {
-#pragma unroll
-            for (int u = 0; u < U; ++u) vec_combine<T>(op, x[gi][u], a[u]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long i = i0 + (long long)u * TT;
-      if (i < nvec) {
-        if (do_scale) acc_scale<T>(a[u], scale);
-        st16(dst + i * 16, acc_to_vec<T>(a[u]));
-      }
-    }
-  }
-  // scalar tail (or the whole step when some pointer is not 16-byte aligned)
-  for (long long e = nvec * VE + g; e < count; e += TT) {
-    Acc a = Elem<T>::up(reinterpret_cast<const T*>(s_ptr[0])[e]);
-    for (int s = 1; s < nsrc; ++s)
-      a = combine<Acc>(op, a, Elem<T>::up(__ldcg(reinterpret_cast<const T*>(s_ptr[s]) + e)));
-    if (do_scale) a = (Acc)(a * scale);
-    reinterpret_cast<T*>(dst)[e] = Elem<T>::down(a);
-  }
+  return a->nsrc >= 0;
 }
 
 // ------------------------------------------------------------------ the kernel
@@ -425,6 +284,43 @@ __device__ __noinline__ RankTables tables_to_smem(const char* __restrict__ blob,
   return t;
 }
 
+// Where a CTA is in the schedule.  In shared memory rather than in registers: nothing of it is then live across the
+// call that runs a span (see run_span).
+struct RoundWalk {
+  const DevRound* rounds;
+  const DevStep* steps;
+  const DevSrc* srcs;
+  const int* order;
+  int nst, nsmall, nb, ord_begin;
+  long long te, nitems;      // tile of the large steps in elements; small steps + tiles
+};
+
+// Tile size: every CTA gets the same number m of tiles (one, unless that tile would exceed kTileMax), each as
+// large as that allows: the shortest chain of dependent round trips per CTA and the most bytes in flight per
+// thread, and no CTA left with one tile more than the others.  A large step is cut into q = nct * m / nb tiles.
+template <typename T>
+__device__ __forceinline__ void walk_round(const DevRound& R, unsigned nct, RoundWalk* k) {
+  k->nst = R.step_end - R.step_begin;
+  k->nb = R.nbig;
+  k->nsmall = k->nst - R.nbig;
+  k->ord_begin = R.ord_begin;
+  const long long grain_e = kTileGrain / (long long)sizeof(T), max_e = kTileMax / (long long)sizeof(T);
+  long long te = kTileMin / (long long)sizeof(T);
+  long long rows = 0;
+  if (R.nbig > 0) {
+    long long m = (R.big_max * R.nbig + (long long)nct * max_e - 1) / ((long long)nct * max_e);
+    if (m < 1) m = 1;
+    long long q = (long long)nct * m / R.nbig;
+    if (q < 1) q = 1;
+    long long t = (R.big_max + q - 1) / q;
+    t = (t + grain_e - 1) / grain_e * grain_e;
+    if (t > te) te = t;
+    rows = (R.big_max + te - 1) / te;
+  }
+  k->te = te;
+  k->nitems = (long long)k->nsmall + rows * R.nbig;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kInterpThreads, 1)
 interp_kernel(World w, const char* __restrict__ blob, IoTable io, int op, float scale, int tables_in_smem) {
@@ -462,11 +358,15 @@ interp_kernel(World w, const char* __restrict__ blob, IoTable io, int op, float 
 
   __shared__ unsigned long long s_base;
   __shared__ int s_ok;
-  __shared__ const char* s_ptr[kMaxSrc + 1];
-  __shared__ int s_meta[4];
+  __shared__ SpanArgs s_span;
+  __shared__ RoundWalk s_walk;
   if (tid == 0) {
     s_base = epoch_first;
     s_ok = abort_first ? 0 : 1;
+    s_walk.rounds = rounds;
+    s_walk.steps = steps;
+    s_walk.srcs = srcs;
+    s_walk.order = order;
   }
   __syncthreads();
   const unsigned long long base = s_base;
@@ -478,53 +378,37 @@ interp_kernel(World w, const char* __restrict__ blob, IoTable io, int op, float 
   bool ok = s_ok != 0;
 
   for (int t = 0; t < nrounds && ok; ++t) {
-    const DevRound R = rounds[t];
-    for (int i = R.wait_begin + tid; i < R.wait_end; i += blockDim.x) {
+    const DevRound* R = s_walk.rounds + t;
+    for (int i = R->wait_begin + tid; i < R->wait_end; i += blockDim.x) {
       const DevWait wt = waits[i];
       if (!wait_flag_ge(&w.sig[rank][wt.peer], base + (unsigned long long)wt.need + 1ull, c, w.timeout_ns,
                         ST_TIMEOUT_ROUND, rank, t, wt.peer))
         s_ok = 0;
     }
+    if (tid == 0) walk_round<T>(*R, nct, &s_walk);
     __syncthreads();
     ok = s_ok != 0;
     if (!ok) break;
     unsigned long long* tr = w.trace[rank];
     if (tr && cta == 0 && tid == 0 && t < w.trace_rounds) tr[2 * t] = globaltimer_ns();   // waits of round t satisfied
-    const int nst = R.step_end - R.step_begin;
-    if (nst > 0) {
-      // Tile size: every CTA gets the same number m of tiles (one, unless that tile would exceed kTileMax), each as
-      // large as that allows: the shortest chain of dependent round trips per CTA and the most bytes in flight per
-      // thread, and no CTA left with one tile more than the others.  A large step is cut into q = nct * m / nb tiles.
-      const int nb = R.nbig, nsmall = nst - nb;
-      const long long grain_e = kTileGrain / (long long)sizeof(T), max_e = kTileMax / (long long)sizeof(T);
-      long long te = kTileMin / (long long)sizeof(T);
-      if (nb > 0) {
-        long long m = (R.big_max * nb + (long long)nct * max_e - 1) / ((long long)nct * max_e);
-        if (m < 1) m = 1;
-        long long q = (long long)nct * m / nb;
-        if (q < 1) q = 1;
-        long long t = (R.big_max + q - 1) / q;
-        t = (t + grain_e - 1) / grain_e * grain_e;
-        if (t > te) te = t;
-      }
-      const long long rows = nb ? (R.big_max + te - 1) / te : 0;
-      const long long nitems = (long long)nsmall + rows * nb;
+    if (s_walk.nst > 0) {
       // work items of this round: the small steps (one CTA each), then the tiles of the large steps
-      for (long long v = cta; v < nitems; v += nct) {
+      for (long long v = cta; v < s_walk.nitems; v += nct) {
         int sidx;
         long long e0 = 0;
-        if (v < nsmall) {
-          sidx = order[R.ord_begin + nb + (int)v];
+        if (v < s_walk.nsmall) {
+          sidx = s_walk.order[s_walk.ord_begin + s_walk.nb + (int)v];
         } else {
-          const long long u = v - nsmall;
-          sidx = order[R.ord_begin + (int)((u % nb + rank) % nb)];
-          e0 = (u / nb) * te;
+          const unsigned u = (unsigned)(v - s_walk.nsmall), nb = (unsigned)s_walk.nb;
+          sidx = s_walk.order[s_walk.ord_begin + (int)((u % nb + (unsigned)rank) % nb)];
+          e0 = (long long)(u / nb) * s_walk.te;
         }
-        const DevStep st = steps[sidx];
+        const DevStep st = s_walk.steps[sidx];
         if (e0 >= st.count) continue;
         long long cnt = st.count - e0;
-        if (v >= nsmall && cnt > te) cnt = te;
-        run_step<T>(st, srcs, w, io, rank, e0, cnt, 0u, 1u, op, scale, s_ptr, s_meta, h->limit);
+        if (v >= s_walk.nsmall && cnt > s_walk.te) cnt = s_walk.te;
+        __syncthreads();      // the readers of the previous span's arguments are done
+        if (set_step<T>(st, s_walk.srcs, w, io, rank, e0, cnt, op, scale, &s_span, h->limit)) run_span<T>(&s_span);
       }
       ok = rank_barrier(c, nct, gen, w.timeout_ns, rank, t);
       if (!ok) break;
@@ -532,12 +416,14 @@ interp_kernel(World w, const char* __restrict__ blob, IoTable io, int op, float 
     // (a round without steps only announces that this rank has entered: nothing to wait for)
     if (tr && cta == 0 && tid == 0 && t < w.trace_rounds) tr[2 * t + 1] = globaltimer_ns();  // round t complete on this rank
     if (cta == 0) {
-      const int n = R.sig_end - R.sig_begin;
+      R = s_walk.rounds + t;
+      const int n = R->sig_end - R->sig_begin;
       for (int i = tid; i < n; i += blockDim.x) {
         __threadfence_system();
-        st_release_sys(&w.sig[sigs[R.sig_begin + i]][rank], base + (unsigned long long)t + 1ull);
+        st_release_sys(&w.sig[sigs[R->sig_begin + i]][rank], base + (unsigned long long)t + 1ull);
       }
     }
+    __syncthreads();          // the walk of this round is no longer read
   }
   // peers that read this rank's caller buffers directly must be done with them
   if (ok) {
