@@ -21,6 +21,11 @@ int chb_run_program(chb_comm* c, const chb_program* p, int dtype, int op, const 
                     void* const* out, float scale, int nctas, cudaStream_t stream);
 int chb_run_program_ll(chb_comm* c, const chb_program* p, int dtype, int op, const void* const* in,
                        void* const* out, float scale, int nctas, cudaStream_t stream);
+int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int op, const void* const* in,
+                             void* const* out, float scale, int nctas, cudaStream_t stream);
+int chb_lockstep_ok(const chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out,
+                    long long slot_bytes);
+int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, long long payload_bytes);
 long long chb_program_ll_lines(const chb_program* p, int esz);
 int chb_ll_collective(chb_comm* c, int mode, int dtype, int op, const void* const* in, void* const* out,
                       long long count, float scale, int nctas, cudaStream_t stream);
@@ -188,6 +193,9 @@ int chb_collective(chb_comm* c, int coll, const char* algo, int k, int b, int au
   // aliased allgather inputs sit at a different heap offset on every rank, so
   // peers cannot address them as "my input pointer, your heap": stage them
   if (ag_alias) flags &= ~1;
+  // Without a suffix, a world whose ranks all live on this GPU runs in lockstep (kernels/lockstep.cu) with the program,
+  // and under the refusals, of the mode it would have run in otherwise.
+  const long long slot = coll == CHB_ALLGATHER ? (long long)count * chb_dtype_size(dtype) : 0;
   chb_program* p = nullptr;
   if (mode != 2 && ll_kind && c->P > 1) {
     static const long long ll_max = [] {
@@ -202,6 +210,9 @@ int chb_collective(chb_comm* c, int coll, const char* algo, int k, int b, int au
       int rc = get_program(c, coll, algo, k, b, aux, count, ll_flags, &p);
       if (rc) return rc;
       const long long need = chb_program_ll_lines(p, esz);
+      if (mode == 0 && need <= (long long)c->P * (long long)c->ll_lines_per_src && chb_lockstep_ok(c, p, dtype, in, out, slot) &&
+          chb_lockstep_beats_push(c, p, dtype, payload))
+        return chb_run_program_lockstep(c, p, dtype, op, in, out, scale, nctas, stream);
       if (need <= (long long)c->P * (long long)c->ll_lines_per_src)
         return chb_run_program_ll(c, p, dtype, op, in, out, scale, nctas, stream);
       if (mode == 1) { c->last_error = "messages of this program exceed the flagged-line inbox"; return CHB_ERR_COUNT; }
@@ -209,6 +220,8 @@ int chb_collective(chb_comm* c, int coll, const char* algo, int k, int b, int au
   }
   int rc = get_program(c, coll, algo, k, b, aux, count, flags, &p);
   if (rc) return rc;
+  if (mode == 0 && chb_lockstep_ok(c, p, dtype, in, out, slot))
+    return chb_run_program_lockstep(c, p, dtype, op, in, out, scale, nctas, stream);
   return chb_run_program(c, p, dtype, op, in, out, scale, nctas, stream);
 }
 

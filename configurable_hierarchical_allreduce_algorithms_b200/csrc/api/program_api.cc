@@ -5,6 +5,7 @@
 #include <string>
 
 #include "../sched/ll_plan.h"
+#include "../sched/lock_plan.h"
 #include "../sched/algos.h"
 #include "../sched/program.h"
 #include "chb.h"
@@ -140,6 +141,28 @@ int chb_program_simulate_ll(const chb_program_t* p, int dtype, int op, void* con
   if (!p || !in || !out || fault < 0 || fault > 2) return CHB_ERR_ARG;
   std::string e;
   int rc = chb::simulate_ll(p->prog, dtype, op, in, out, seed, nthreads, fault, launches, &e);
+  if (rc) { set_err(err, errlen, e); return rc == -1 ? CHB_ERR_TIMEOUT : CHB_ERR_ARG; }
+  return CHB_SUCCESS;
+}
+
+// The lockstep form (all ranks of the program run by one grid): rounds, steps and remaining destinations after the
+// rewriting, and the same without it.
+int chb_program_lock_info(const chb_program_t* p, int rewrite, long long* info, int n) {
+  if (!p || !info) return CHB_ERR_ARG;
+  if (rewrite < chb::LOCK_PLAIN || rewrite > chb::LOCK_CHAINS) return CHB_ERR_ARG;
+  const chb::LockPlan plan = chb::make_lock_plan(p->prog, rewrite);
+  long long reads = 0, stores = 0;
+  for (const chb::LockStepPlan& x : plan.steps) { reads += x.count * (long long)x.srcs.size(); stores += x.count * (long long)x.dsts.size(); }
+  const long long v[4] = {plan.nrounds, (long long)plan.steps.size(), reads, stores};
+  for (int i = 0; i < n && i < 4; ++i) info[i] = v[i];
+  return CHB_SUCCESS;
+}
+
+int chb_program_simulate_lock(const chb_program_t* p, int dtype, int op, void* const* in, void* const* out,
+                              uint64_t seed, int rewrite, char* err, int errlen) {
+  if (!p || !in || !out || rewrite < chb::LOCK_PLAIN || rewrite > chb::LOCK_CHAINS) return CHB_ERR_ARG;
+  std::string e;
+  const int rc = chb::simulate_lock(p->prog, dtype, op, in, out, seed, rewrite, &e);
   if (rc) { set_err(err, errlen, e); return rc == -1 ? CHB_ERR_TIMEOUT : CHB_ERR_ARG; }
   return CHB_SUCCESS;
 }

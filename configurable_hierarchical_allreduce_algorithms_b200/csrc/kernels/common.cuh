@@ -63,6 +63,12 @@ struct World {
   int reserved2;
 };
 
+// Caller buffers of every rank (peers' entries only where a step program reads them).
+struct IoTable {
+  const char* in[kMaxRanks];
+  char* out[kMaxRanks];
+};
+
 // ------------------------------------------------------------------ PTX helpers
 __device__ __forceinline__ unsigned long long ld_acquire_sys(const unsigned long long* p) {
   unsigned long long v;

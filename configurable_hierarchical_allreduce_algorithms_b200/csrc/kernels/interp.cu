@@ -46,14 +46,9 @@ constexpr long long kDevRanksOffset = 128;
 static_assert(sizeof(DevHeader) <= kDevRanksOffset, "the rank table starts right after the header");
 constexpr long long kInterpSmemTables = 40 << 10;   // bytes of table entries a CTA keeps in shared memory
 
-struct IoTable {
-  const char* in[kMaxRanks];
-  char* out[kMaxRanks];
-};
-
 // Every range a program touches lies inside the buffer it names: checked once per program before
 // its schedule is uploaded, so that a generator bug cannot turn into a stray peer access.
-static bool ranges_ok(const Program& p, std::string* why) {
+bool program_ranges_ok(const Program& p, std::string* why) {
   const int64_t lim[3] = {p.in_elems, p.out_elems, p.work_elems};
   for (size_t i = 0; i < p.ops.size(); ++i) {
     const Op& o = p.ops[i];
@@ -497,7 +492,7 @@ static int get_blob(chb_comm* c, const chb_program* p, void** out) {
   auto it = c->blobs.find(p->uid);
   if (it != c->blobs.end()) { *out = it->second; return CHB_SUCCESS; }
   if (p->prog.stats.max_nsrc > kMaxSrc) { c->last_error = "program has a step with too many sources"; return CHB_ERR_UNSUPPORTED; }
-  if (!ranges_ok(p->prog, &c->last_error)) return CHB_ERR_ARG;
+  if (!program_ranges_ok(p->prog, &c->last_error)) return CHB_ERR_ARG;
   long long table_bytes = 0;
   std::vector<char> blob = make_blob(p->prog, &table_bytes);
   void* d = nullptr;
@@ -524,6 +519,10 @@ void chb_program_release(chb_comm* c, const chb_program* p) {
   if (!p) return;
   auto it = c->blobs.find(p->uid);
   if (it != c->blobs.end()) { cudaFree(it->second); c->blobs.erase(it); c->blob_table_bytes.erase(p->uid); }
+  for (uint64_t key = p->uid * 2u; key < p->uid * 2u + 2u; ++key) {
+    auto lt = c->lock_blobs.find(key);
+    if (lt != c->lock_blobs.end()) { cudaFree(lt->second.dev); c->lock_blobs.erase(lt); }
+  }
   for (auto jt = c->ll_blobs.lower_bound(p->uid * 16u); jt != c->ll_blobs.end() && jt->first < (p->uid + 1) * 16u;) {
     cudaFree(jt->second.first);
     jt = c->ll_blobs.erase(jt);

@@ -89,10 +89,10 @@ __device__ __forceinline__ void reduce_loop32(const char* const* src, long long 
   }
 }
 
-// Plain copy of 256-bit vectors (gather / broadcast steps, staging): no arithmetic, UC vectors in flight per thread.
-// Whole groups only; returns this thread's first vector that is left.
+// Plain copy of 256-bit vectors (gather / broadcast steps, staging): no arithmetic (the bits stay, whatever they
+// encode), UC vectors in flight per thread, what is left one by one.
 template <int UC>
-__device__ __forceinline__ int copy_loop32(const char* src, char* const* dst, int ndst, long long dofs, int j0, int nw, int TT) {
+__device__ __forceinline__ void copy_loop32(const char* src, char* const* dst, int ndst, long long dofs, int j0, int nw, int TT) {
   const int stride = TT * 32;
 #pragma unroll 1
   for (; j0 + (UC - 1) * TT < nw; j0 += TT * UC) {
@@ -107,7 +107,13 @@ __device__ __forceinline__ int copy_loop32(const char* src, char* const* dst, in
       for (int u = 0; u < UC; ++u) st32(q + u * stride, lo[u], hi[u]);
     }
   }
-  return j0;
+#pragma unroll 1
+  for (; j0 < nw; j0 += TT) {
+    uint4 lo, hi;
+    ld32_cg(src + (long long)j0 * 32, lo, hi);
+#pragma unroll 1
+    for (int d = 0; d < ndst; ++d) st32(dst[d] + dofs + (long long)j0 * 32, lo, hi);
+  }
 }
 
 // Bytes [sh, sh + 16) of the 32 bytes {lo, hi}, 0 < sh < 16 (the same sh in all lanes).
@@ -197,6 +203,49 @@ __device__ __forceinline__ void reduce_loop16(const char* const* src, int nsrc, 
   }
 }
 
+// The same for a plain copy.
+template <int U>
+__device__ __forceinline__ void copy_loop16(const char* src, char* const* dst, int ndst, long long pos, long long nv) {
+  const int lane = threadIdx.x & 31;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  const char* p = src + pos;
+  const unsigned sh = (unsigned)(reinterpret_cast<unsigned long long>(p) & 15ull);
+  p -= sh;
+  const long long words = nv + (sh ? 1 : 0);
+  const long long step = (long long)(blockDim.x >> 5) * 32 * U;
+#pragma unroll 1
+  for (long long base = (long long)(threadIdx.x >> 5) * 32 * U; base < nv; base += step) {   // uniform per warp
+    uint4 x[U], tail = zero;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long j = base + u * 32 + lane;
+      x[u] = zero;
+      if (j < words) x[u] = ld16_cg(p + j * 16);
+    }
+    if (sh && lane == 31 && base + U * 32 < words) tail = ld16_cg(p + (base + U * 32) * 16);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      uint4 v = x[u];
+      if (sh) {
+        const uint4 give = (lane == 0 && u + 1 < U) ? x[u + 1 < U ? u + 1 : u] : v;
+        const int from = (lane + 1) & 31;
+        uint4 next;
+        next.x = __shfl_sync(0xffffffffu, give.x, from);
+        next.y = __shfl_sync(0xffffffffu, give.y, from);
+        next.z = __shfl_sync(0xffffffffu, give.z, from);
+        next.w = __shfl_sync(0xffffffffu, give.w, from);
+        if (u + 1 == U && lane == 31) next = tail;
+        v = funnel16(v, next, sh);
+      }
+      const long long j = base + u * 32 + lane;
+      if (j < nv) {
+#pragma unroll 1
+        for (int d = 0; d < ndst; ++d) st16(dst[d] + pos + j * 16, v);
+      }
+    }
+  }
+}
+
 // One span: dst[d][e] = scale * (src[0][e] op src[1][e] op ...) for e < count.  All threads of the CTA; src / dst are
 // in shared memory; the destinations are equal modulo 16 (the caller issues one span for each otherwise).
 // A source may be a destination as well (same address, same element): every element is loaded by the thread that
@@ -218,9 +267,9 @@ __device__ __forceinline__ void reduce_span(const char* const* src, int nsrc, ch
     if (lo > bytes) lo = bytes;
     const int nw = (int)((bytes - lo) / 32);       // (a span is far below 2^31 vectors)
     hi = lo + (long long)nw * 32;
-    int j0 = tid;
-    if (plain) j0 = copy_loop32<4>(src[0] + lo, dst, ndst, lo, j0, nw, nt);
-    if (op != OP_SUM) reduce_loop32<T, false, 2, 1>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
+    const int j0 = tid;
+    if (plain) copy_loop32<4>(src[0] + lo, dst, ndst, lo, j0, nw, nt);
+    else if (op != OP_SUM) reduce_loop32<T, false, 2, 1>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
     else if (nw <= nt) reduce_loop32<T, true, G1, 1>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
     else reduce_loop32<T, true, G2, U2>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
   } else {
@@ -231,19 +280,20 @@ __device__ __forceinline__ void reduce_span(const char* const* src, int nsrc, ch
     const long long left = bytes - lo - room;
     const long long nv = left > 0 ? left / 16 : 0;
     hi = lo + nv * 16;
-    if (op == OP_SUM) reduce_loop16<T, true, 2, kUnroll16<T>>(src, nsrc, dst, ndst, lo, nv, op, do_scale, scale);
+    if (plain) copy_loop16<4>(src[0], dst, ndst, lo, nv);
+    else if (op == OP_SUM) reduce_loop16<T, true, 2, kUnroll16<T>>(src, nsrc, dst, ndst, lo, nv, op, do_scale, scale);
     else reduce_loop16<T, false, 2, 1>(src, nsrc, dst, ndst, lo, nv, op, do_scale, scale);
   }
-  // both ends, element by element
+  // both ends, element by element (by the last threads: in a short span they had no vector and start at once)
   const int head = (int)(lo / (long long)sizeof(T));
   const long long at = hi / (long long)sizeof(T);
   const int edge = head + (int)(count - at);
-  for (int i = tid; i < edge; i += nt) {
+  for (int i = nt - 1 - tid; i < edge; i += nt) {
     const long long e = i < head ? i : at + (i - head);
     Acc a = Elem<T>::up(__ldcg(reinterpret_cast<const T*>(src[0]) + e));
     for (int s = 1; s < nsrc; ++s) a = combine<Acc>(op, a, Elem<T>::up(__ldcg(reinterpret_cast<const T*>(src[s]) + e)));
     if (do_scale) a = (Acc)(a * scale);
-    const T v = Elem<T>::down(a);
+    const T v = plain ? __ldcg(reinterpret_cast<const T*>(src[0]) + e) : Elem<T>::down(a);
     for (int d = 0; d < ndst; ++d) reinterpret_cast<T*>(dst[d])[e] = v;
   }
 }

@@ -1,0 +1,66 @@
+// The lockstep form of a lowered step program: what kernels/lockstep.cu executes when one launch runs ALL ranks on
+// one GPU.
+//
+// Nobody has to be signalled there: every CTA can execute steps of any rank, one barrier over the whole grid separates
+// two rounds, and every buffer is visible to every step.  So the program is rewritten as plain data flow before it is
+// laid out:
+//   1. a step that reads what an earlier copy wrote (staging, a broadcast hop) reads that copy's source instead;
+//   2. a copy of what an earlier step produced becomes one more destination of that step;
+//   3. a reduction that only continues another one takes over its operands (a ring or pairwise chain becomes one step):
+//      where the accumulator is the stored type, so that no rounding falls out;
+//   4. writes that nobody reads any more are dropped (scratch, and what a later step replaces);
+//   5. rounds are assigned anew, and copies of one source within a round become one step with several destinations.
+// Steps are cut where a reader needs a part of what a writer produced.  Every rewrite keeps the serial meaning of the
+// program (it is refused when a step in between touches the memory concerned), the order in which a reduction combines
+// its operands, and the rounding between two steps, so results are the pull form's bit for bit.
+#pragma once
+#include <cstdint>
+#include <string>
+#include <vector>
+
+#include "program.h"
+
+namespace chb {
+
+constexpr int kLockMaxDst = 16;          // destinations of one step
+constexpr size_t kLockMaxSrc = 40;       // sources of one step
+constexpr int64_t kLockGrain = 2048;     // elements: the unit in which a round's work is dealt to the CTAs
+constexpr size_t kLockMaxRewrite = 512;  // longer programs are laid out as they are (the rewriting compares steps pairwise)
+
+struct LockDst { int32_t rank, buf; int64_t off; };
+struct LockStepPlan {
+  int64_t count = 0;
+  bool final = false;               // the reduction's scale applies here
+  int32_t level = 0;
+  std::vector<Src> srcs;            // an accumulate operand is the first source
+  std::vector<LockDst> dsts;
+};
+struct LockPlan {
+  int P = 0, nrounds = 0;
+  int64_t in_elems = 0, out_elems = 0, work_elems = 0;
+  std::vector<LockStepPlan> steps;  // ordered by round
+};
+
+// rewrite: LOCK_PLAIN only the layout (for comparing), LOCK_COPIES without rewrite 3, LOCK_CHAINS everything.
+enum { LOCK_PLAIN = 0, LOCK_COPIES = 1, LOCK_CHAINS = 2 };
+// The rewriting for a stored type: 16-bit floats are rounded after every step, the others accumulate in themselves
+// (bytes in 32 bits, which agrees modulo 256).
+inline int lock_rewrite_for(int dtype) { return dtype == DT_BF16 || dtype == DT_F16 ? LOCK_COPIES : LOCK_CHAINS; }
+LockPlan make_lock_plan(const Program& p, int rewrite);
+
+// Device tables: LockHeader, LockRound[nrounds], LockStep[nsteps], LockRef[nrefs] (a step's sources, then its
+// destinations).  prefix: cost of the round's earlier steps; the cost of a step is its grains x (sources + destinations).
+// elems: elements of the round's earlier steps.
+struct LockHeader { int nrounds, nsteps, nrefs, pad; };
+struct LockRound { int step_begin, step_end; long long cost, elems, pad; };
+struct LockStep { long long prefix, count, elems; int ref_begin, nsrc, ndst, final, pad0, pad1; };
+struct LockRef { long long off; int rank, buf; };
+static_assert(sizeof(LockHeader) % 16 == 0 && sizeof(LockRound) % 16 == 0 && sizeof(LockStep) % 16 == 0 && sizeof(LockRef) % 16 == 0, "copied as 16-byte words");
+std::vector<char> make_lock_blob(const LockPlan& p);
+
+// Executes the plan on host memory, the steps of a round in random order, and checks that no step of a round touches
+// what another one writes.  Returns 0, -1 (err says what) or -2 for a bad argument.
+int simulate_lock(const Program& p, int dtype, int op, void* const* in, void* const* out, uint64_t seed,
+                  int rewrite, std::string* err);
+
+}  // namespace chb

@@ -120,6 +120,7 @@ Program Builder::lower(const LowerOpts& o) const {
   p.out_elems = out_elems_;
   p.in_symmetric = o.in_symmetric;
   p.out_symmetric = o.out_symmetric;
+  p.in_place = o.in_place;
 
   // ---- 1. which caller buffers do peers read? --------------------------------
   bool rin = false, rout = false;

@@ -82,7 +82,7 @@ struct Program {
   int P = 0;
   int64_t in_elems = 0, out_elems = 0, work_elems = 0;
   int nrounds = 0;
-  bool in_symmetric = false, out_symmetric = false;
+  bool in_symmetric = false, out_symmetric = false, in_place = false;
   bool reads_peer_in = false, reads_peer_out = false;
   std::vector<Op> ops;                          // physical buffers, level set
   std::vector<std::vector<RankRound>> rr;       // [rank][round]

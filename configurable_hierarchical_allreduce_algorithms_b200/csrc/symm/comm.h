@@ -43,6 +43,10 @@ struct chb_comm {
   // flagged-line form of compiled programs: key = program id * 16 + element size; value = device tables
   // and the line count of the busiest level (sizes the grid)
   std::map<uint64_t, std::pair<void*, std::pair<long long, long long>>> ll_blobs;   // blob, (busiest level lines, largest rank table bytes)
+  // lockstep form of compiled programs (emulated worlds), by 2 * program id + rewriting: grains of the busiest round, element loads and
+  // stores in all, the bits set in any offset or length
+  struct LockBlob { void* dev = nullptr; int bytes = 0, nrefs = 0, nrounds = 0, saved_rounds = 0; long long max_grains = 0, accesses = 0, grid = 0; };
+  std::map<uint64_t, LockBlob> lock_blobs;
   std::string last_error;
   // set only by the native constructors (chb_comm_create_ipc / chb_comm_create_emulated), which own the heap
   void* owned_heap = nullptr;
@@ -62,6 +66,12 @@ struct chb_comm {
     return heap[peer] + (c - b);
   }
 };
+
+namespace chb {
+struct Program;
+// Every range a program touches lies inside the buffer it names (kernels/interp.cu).
+bool program_ranges_ok(const Program& p, std::string* why);
+}
 
 // CHB_TABLES_IN_SMEM=0 keeps the program kernels' schedule tables in global memory (for A/B timing and debugging)
 inline bool tables_in_smem_wanted() {

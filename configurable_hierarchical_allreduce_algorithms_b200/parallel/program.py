@@ -169,6 +169,38 @@ class Program:
             raise RuntimeError(f"simulate({self.name}) failed: {err.value.decode()}")
         return [o[:self.out_elems] for o in outs]
 
+    def simulate_lock(self, inputs: list[np.ndarray], op: str = "sum", seed: int = 0, rewrite: int = 2,
+                      alias: bool = False) -> list[np.ndarray]:
+        """Run the lockstep form (all ranks executed by one grid, ``csrc/sched/lock_plan.h``) on host arrays, the steps
+        of a round in random order.  ``rewrite``: 0 leaves the program's steps as lowered, 1 rewrites copies, 2 also joins
+        chains of reductions; ``alias`` as in :meth:`simulate`."""
+        assert len(inputs) == self.P
+        dt = np.dtype(inputs[0].dtype)
+        poison = 239 if dt.kind == "u" else -17
+        if alias:
+            assert self.in_place, "aliased buffers need a program lowered with in_place=True"
+            ins = outs = [np.full(max(self.in_elems, self.out_elems), poison, dtype=dt) for _ in range(self.P)]
+            for buf, x in zip(ins, inputs):
+                buf[:x.size] = x
+        else:
+            ins = [np.ascontiguousarray(x, dtype=dt) for x in inputs]
+            outs = [np.full(self.out_elems, poison, dtype=dt) for _ in range(self.P)]
+        ip = (C.c_void_p * self.P)(*[x.ctypes.data for x in ins])
+        opp = (C.c_void_p * self.P)(*[x.ctypes.data for x in outs])
+        err = C.create_string_buffer(512)
+        rc = N.lib().chb_program_simulate_lock(self._h, _DT_FROM_NP[dt], _OPS[op], ip, opp, seed, int(rewrite), err, len(err))
+        if rc:
+            raise RuntimeError(f"simulate_lock({self.name}) failed: {err.value.decode()}")
+        return [o[:self.out_elems] for o in outs]
+
+    def lock_info(self, rewrite: int = 2) -> dict:
+        """Rounds, steps, elements read and elements stored of the lockstep form."""
+        v = (C.c_longlong * 4)()
+        rc = N.lib().chb_program_lock_info(self._h, int(rewrite), v, 4)
+        if rc:
+            raise RuntimeError(f"lock_info failed with code {rc}")
+        return dict(zip(("rounds", "steps", "reads", "stores"), [int(x) for x in v]))
+
     def simulate_ll(self, inputs: list[np.ndarray], op: str = "sum", seed: int = 0, threads: int = 5,
                     fault: int = 0, launches: int = 1) -> list[np.ndarray]:
         """Run the push (flagged-line) form of this program on host arrays, line by line, the way the GPU executor

@@ -1,0 +1,101 @@
+"""All ranks of an emulated world in one grid (the way a schedule without an execution-mode suffix runs there), against
+the pull interpreter: bit for bit, on floats that do not add exactly, for aligned and odd lengths, skewed buffers, in
+place, and mixed with the per-rank kernels on one communicator."""
+import pytest
+import torch
+
+import configurable_hierarchical_allreduce_algorithms_b200 as chb
+from configurable_hierarchical_allreduce_algorithms_b200.parallel.comm import Communicator
+
+pytestmark = pytest.mark.gpu
+
+FNS = {"allreduce": chb.all_reduce, "reduce_scatter": chb.reduce_scatter, "allgather": chb.all_gather, "alltoall": chb.all_to_all}
+
+
+def lengths(coll, P, n):
+    return {"allreduce": (n * P, n * P), "reduce_scatter": (n * P, n), "allgather": (n, n * P), "alltoall": (n * P, n * P)}[coll]
+
+
+@pytest.mark.parametrize("P,k,b", [(2, 2, 1), (3, 2, 1), (8, 2, 1), (8, 4, 2), (8, 2, 4), (6, 3, 2), (16, 4, 4)])
+@pytest.mark.parametrize("coll", list(FNS))
+def test_lockstep_equals_pull(cuda, coll, P, k, b):
+    comm = Communicator.emulated(P, ll_bytes=64 << 10, scratch_bytes=16 << 20, user_bytes=4096)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    names = ["tuna", "linear"] if coll == "alltoall" else ["radix_batch", "ring"]
+    # one element, a grain of 2048 elements and its neighbours, several grains with a rest
+    for i, n in enumerate((1, 31, 2047, 2048, 2049, 40013)):
+        for dtype in (torch.float32, torch.bfloat16) if n > 1 else (torch.float32, torch.float64, torch.uint8):
+            n_in, n_out = lengths(coll, P, n)
+            skew = [(i + r * (i % 2)) % 3 for r in range(P)]      # ranks on different 16-byte grids every second time
+            src = [torch.rand(n_in + 4, generator=g, device="cuda").mul_(9).to(dtype) for _ in range(P)]
+            ins = [s[a:a + n_in] for s, a in zip(src, skew)]
+            full = [torch.zeros(n_out + 4, dtype=dtype, device="cuda") for _ in range(P)]
+            outs = [f[a:a + n_out] for f, a in zip(full, skew)]
+            for name in names:
+                kw = dict(k=k, b=b)
+                if coll in ("allreduce", "reduce_scatter") and dtype.is_floating_point:
+                    kw["scale"] = 0.37
+                want = FNS[coll](comm, ins, algo=name + ":pull", **kw)
+                for f in full:
+                    f.zero_()
+                FNS[coll](comm, ins, out=outs, algo=name, **kw)
+                for r in range(P):
+                    assert torch.equal(outs[r], want[r]), (name, n, dtype, r)
+                    assert not full[r][:skew[r]].any() and not full[r][skew[r] + n_out:].any()     # nothing around it
+    comm.check()
+    comm.close()
+
+
+def test_lockstep_in_place_and_overlapping_buffers(cuda):
+    P, n = 4, 5003
+    comm = Communicator.emulated(P, scratch_bytes=4 << 20, user_bytes=4096)
+    src = [torch.randn(n * P, device="cuda") for _ in range(P)]
+    want = chb.all_reduce(comm, src, algo="radix_batch:pull", k=2, b=2)
+    bufs = [s.clone() for s in src]
+    chb.all_reduce(comm, bufs, out=bufs, algo="radix_batch", k=2, b=2)
+    assert all(torch.equal(x, y) for x, y in zip(bufs, want))
+    # reduce-scatter into the rank's own block of its input: known to no schedule, so it stays with the interpreter
+    want = chb.reduce_scatter(comm, src, algo="radix_batch:pull")
+    bufs = [s.clone() for s in src]
+    outs = chb.reduce_scatter(comm, bufs, out=[b[r * n:(r + 1) * n] for r, b in enumerate(bufs)], algo="radix_batch")
+    assert all(torch.equal(x, y) for x, y in zip(outs, want))
+    # allgather of blocks that already lie in their slots
+    full = [torch.zeros(n * P, device="cuda") for _ in range(P)]
+    for r in range(P):
+        full[r][r * n:(r + 1) * n] = src[r][:n]
+    chb.all_gather(comm, [f[r * n:(r + 1) * n] for r, f in enumerate(full)], out=full, algo="radix_batch", k=2, b=2)
+    cat = torch.cat([s[:n] for s in src])
+    assert all(torch.equal(f, cat) for f in full)
+    comm.check()
+    comm.close()
+
+
+def test_lockstep_mixes_with_the_per_rank_kernels(cuda):
+    """Launch counters, epochs and sequence numbers: lockstep, pull, push and one-shot launches in any order, traced
+    launches in between, and replays of a captured launch."""
+    P, n = 8, 8 * 1000
+    comm = Communicator.emulated(P, scratch_bytes=4 << 20, user_bytes=4096)
+    src = [torch.randint(-9, 9, (n,), device="cuda", dtype=torch.int32) for _ in range(P)]
+    want = torch.stack(src).sum(0)
+    outs = [torch.zeros_like(s) for s in src]
+    before = comm.status(5)["launches"]
+    for i in range(3):
+        for algo in ("radix_batch", "radix_batch:pull", "ring", "ll", "radix_batch:ll", "recursive_doubling"):
+            chb.all_reduce(comm, src, out=outs, algo=algo, k=2, b=4)
+            assert all(torch.equal(o, want) for o in outs), algo
+    assert comm.status(5)["launches"] - before == 18
+    comm.enable_trace(16)                                   # stamps describe ranks that signal each other
+    chb.all_reduce(comm, src, out=outs, algo="recursive_doubling")
+    assert comm.read_trace(2, 3)[-1][1] > 0
+    comm.enable_trace(0)
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        chb.all_reduce(comm, src, out=outs, algo="radix_batch", k=2, b=4, stream=side)
+    for i in range(3):
+        src[0].add_(1)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(outs[6], torch.stack(src).sum(0))
+    comm.check()
+    comm.close()

@@ -1,0 +1,56 @@
+"""The lockstep form of a step program (one grid runs all ranks): its rewriting (copies read through, copies folded into
+the step that produces their data, dead scratch dropped, rounds assigned anew) gives the pull form's results bit for bit,
+on float inputs that do not add exactly, for every algorithm and every lowering, with the steps of a round in any order."""
+import numpy as np
+import pytest
+
+import configurable_hierarchical_allreduce_algorithms_b200 as chb
+
+CASES = [(coll, algo) for coll in ("allreduce", "reduce_scatter", "allgather", "alltoall", "gather")
+         for algo in chb.list_algorithms(coll)]
+LOWERINGS = [dict(), dict(in_symmetric=True), dict(out_symmetric=True), dict(in_symmetric=True, out_symmetric=True),
+             dict(in_place=True)]
+
+
+@pytest.mark.parametrize("coll,algo", CASES)
+def test_lockstep_equals_the_pull_form(coll, algo):
+    rng = np.random.default_rng(11)
+    ran = 0
+    for P, k, b in ((2, 2, 1), (3, 2, 1), (4, 2, 2), (6, 2, 3), (6, 3, 2), (8, 2, 1), (8, 2, 4), (8, 4, 2), (8, 8, 8), (5, 4, 1), (12, 3, 4)):
+        for n in (1, 37):
+            count = n * P if coll == "allreduce" else n
+            for low in LOWERINGS:
+                if low.get("in_place") and coll not in ("allreduce", "alltoall"):
+                    continue            # one buffer as input and output: equal lengths
+                try:
+                    p = chb.Program(coll, algo, P, count, k, b, **low)
+                except ValueError:
+                    continue
+                ins = [rng.standard_normal(p.in_elems).astype(np.float32) for _ in range(P)]
+                alias = bool(low.get("in_place"))
+                want = p.simulate([x.copy() for x in ins], alias=alias)
+                for rewrite in (0, 1, 2):
+                    got = p.simulate_lock(ins, seed=ran, rewrite=rewrite, alias=alias)
+                    for r in range(P if coll != "gather" else 1):
+                        assert got[r].tobytes() == want[r].tobytes(), (P, k, b, n, low, rewrite, r)
+                ran += 1
+    assert ran
+
+
+def test_rewriting_removes_the_passes_it_is_for():
+    # flat allreduce: every element read once from each rank and stored once on each, in one round
+    P, n = 8, 8 * 100
+    for low in (dict(), dict(in_symmetric=True, out_symmetric=True)):
+        i = chb.Program("allreduce", "radix_batch", P, n, 2, 1, **low).lock_info()
+        assert (i["rounds"], i["reads"], i["stores"]) == (1, P * n, P * n), (low, i)
+    # allgather: every block read once
+    i = chb.Program("allgather", "radix_batch", P, 100, 2, 1).lock_info()
+    assert (i["rounds"], i["reads"], i["stores"]) == (1, P * 100, P * P * 100)
+    # hierarchical allreduce: rounds and traffic of the reductions only
+    p = chb.Program("allreduce", "radix_batch", P, n, 2, 4)
+    assert p.lock_info()["rounds"] < p.lock_info(rewrite=0)["rounds"]
+    assert p.lock_info()["stores"] < p.lock_info(rewrite=0)["stores"] // 2 + P * n
+    # a pairwise and a ring reduce-scatter add in a chain: one step a rank where nothing is rounded in between
+    for algo in ("pairwise", "ring"):
+        i = chb.Program("reduce_scatter", algo, P, 100, 2, 1).lock_info()
+        assert (i["rounds"], i["reads"], i["stores"]) == (1, P * P * 100, P * 100), (algo, i)
