@@ -403,7 +403,7 @@ interp_kernel(World w, const char* __restrict__ blob, IoTable io, int op, float 
         long long cnt = st.count - e0;
         if (v >= s_walk.nsmall && cnt > s_walk.te) cnt = s_walk.te;
         __syncthreads();      // the readers of the previous span's arguments are done
-        if (set_step<T>(st, s_walk.srcs, w, io, rank, e0, cnt, op, scale, &s_span, h->limit)) run_span<T>(&s_span);
+        if (set_step<T>(st, s_walk.srcs, w, io, rank, e0, cnt, op, scale, &s_span, h->limit)) run_span<T, OneCta<T>>(&s_span);
       }
       ok = rank_barrier(c, nct, gen, w.timeout_ns, rank, t);
       if (!ok) break;

@@ -32,7 +32,6 @@
 
 namespace chb {
 
-constexpr int kLockThreads = 512;
 constexpr int kTinyThreads = 1024;
 constexpr long long kTinyAccesses = 8192;          // loads + stores a round, on average, up to which one CTA runs the schedule
 constexpr int kLockCluster = 8;                    // CTAs of a cluster launch
@@ -159,8 +158,8 @@ lock_tiny_kernel(World w, const char* __restrict__ blob, int blob_bytes, IoTable
 
 // CLUSTER: the grid is one cluster (small messages), else the CTAs are co-resident by a cooperative launch, or the schedule
 // has one round only.
-template <typename T, bool CLUSTER>
-__global__ void __launch_bounds__(kLockThreads, 1)
+template <typename T, bool CLUSTER, typename Shape>
+__global__ void __launch_bounds__(Shape::kThreads, Shape::kPerSm)
 lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem, IoTable io, int op, float scale) {
   extern __shared__ __align__(16) unsigned char lock_tables[];
   __shared__ SpanArgs s_span;
@@ -175,7 +174,7 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
   if (in_smem) {      // one latency for the whole schedule instead of a chain of dependent loads a round
     const uint4* g = reinterpret_cast<const uint4*>(blob);
     uint4* s = reinterpret_cast<uint4*>(lock_tables);
-    for (int i = tid; i < blob_bytes / 16; i += kLockThreads) s[i] = g[i];
+    for (int i = tid; i < blob_bytes / 16; i += Shape::kThreads) s[i] = g[i];
     tab = reinterpret_cast<const char*>(lock_tables);
   }
   __syncthreads();
@@ -239,7 +238,7 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
   // The step in which this CTA's share of a round begins (visible after the next barrier of the CTA).
   auto find_first = [&](const LockRound& R) {
     const long long lo = R.cost * cta / nct;
-    for (int i = R.step_begin + tid; i < R.step_end; i += kLockThreads)
+    for (int i = R.step_begin + tid; i < R.step_end; i += Shape::kThreads)
       if (steps[i].prefix <= lo && (i + 1 == R.step_end || steps[i + 1].prefix > lo)) s_first = i;
   };
   const int nrounds = ok ? h->nrounds : 0;
@@ -256,7 +255,7 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
           if (tid == 0) { s_span.dst[0] = s_dst[d]; s_span.ndst = 1; }
           __syncthreads();
         }
-        run_span<T>(&s_span);
+        run_span<T, Shape>(&s_span);
       }
       __syncthreads();                       // the span's arguments are no longer read
       i = next_share(rounds[t], i + 1);
@@ -276,9 +275,10 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
   });
 }
 
-struct LockKernels { const void *wide, *cluster, *tiny, *tiny_vec; };
+struct LockKernels { const void *wide, *wide2, *cluster, *tiny, *tiny_vec; };
 template <typename T>
-static LockKernels lock_kernels() { return {(const void*)lock_kernel<T, false>, (const void*)lock_kernel<T, true>, (const void*)lock_tiny_kernel<T, false>,
+static LockKernels lock_kernels() { return {(const void*)lock_kernel<T, false, OneCta<T>>, (const void*)lock_kernel<T, false, TwoCtas<T>>,
+          (const void*)lock_kernel<T, true, OneCta<T>>, (const void*)lock_tiny_kernel<T, false>,
           (const void*)lock_tiny_kernel<T, true>}; }
 static LockKernels pick_lock(int dtype) {
   switch (dtype) {
@@ -290,7 +290,7 @@ static LockKernels pick_lock(int dtype) {
     case DT_I64: return lock_kernels<int64_t>();
     case DT_U8: return lock_kernels<uint8_t>();
   }
-  return {nullptr, nullptr, nullptr, nullptr};
+  return {nullptr, nullptr, nullptr, nullptr, nullptr};
 }
 
 }  // namespace chb
@@ -333,10 +333,12 @@ static int get_lock_blob(chb_comm* c, const chb_program* p, int dtype, const chb
     if (!program_ranges_ok(g, &c->last_error)) return CHB_ERR_ARG;
     const LockPlan plan = make_lock_plan(g, rewrite);
     chb_comm::LockBlob b;
-    long long grains = 0;
+    long long grains = 0, cost = 0;
     for (size_t i = 0; i < plan.steps.size(); ++i) {
-      if (i == 0 || plan.steps[i].level != plan.steps[i - 1].level) grains = 0;
+      if (i == 0 || plan.steps[i].level != plan.steps[i - 1].level) grains = cost = 0;
       const long long refs = (long long)(plan.steps[i].srcs.size() + plan.steps[i].dsts.size());
+      cost += (plan.steps[i].count + kLockGrain - 1) / kLockGrain * refs;
+      b.max_cost = cost > b.max_cost ? cost : b.max_cost;
       b.accesses += plan.steps[i].count * refs;
       b.nrefs += (int)refs;
       b.grid |= plan.steps[i].count;
@@ -393,7 +395,12 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
   IoTable io{};
   for (int l = 0; l < c->P; ++l) { io.in[l] = (const char*)in[l]; io.out[l] = (char*)out[l]; }
   long long n = nctas > 0 ? (long long)nctas * c->P : b.max_grains;      // one grain is the least a CTA can be given
-  if (n > c->max_ctas) n = c->max_ctas;
+  // Two CTAs an SM pay where an SM has 512 KiB to move in a round; below that the larger barrier costs more (8 ranks, one
+  // and two: reduce-scatter of odd bf16 blocks, 1.3 MiB an SM, 77 and 67 us; allreduce 4 MiB k = 4, b = 2, 0.3 MiB an SM,
+  // 21 and 25 us).
+  const bool two = nctas <= 0 && b.max_cost * kLockGrain * (long long)esz >= ((long long)c->max_ctas << 19);
+  const long long most = (long long)c->max_ctas * (two ? 2 : 1);
+  if (n > most) n = most;
   if (n < 1) n = 1;
   World w = c->world;
   const char* bp = (const char*)b.dev;
@@ -410,6 +417,8 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
   } else {
     void* args[] = {&w, &bp, &bytes, &in_smem, &io, &op, &scale};
     const size_t smem = in_smem ? (size_t)b.bytes : 0;
+    const void* wide = two ? fn.wide2 : fn.wide;
+    const dim3 block(two ? TwoCtas<float>::kThreads : OneCta<float>::kThreads);
     const bool cluster = b.nrounds > 1 && n > 1 && (n <= kLockCluster || (nctas <= 0 && b.max_grains <= kClusterGrains));
     if (cluster) {
       cudaLaunchConfig_t cfg{};
@@ -418,16 +427,16 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
       attr.val.clusterDim.x = (unsigned)(n < kLockCluster ? n : kLockCluster);
       attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
       cfg.gridDim = dim3(attr.val.clusterDim.x);
-      cfg.blockDim = dim3(kLockThreads);
+      cfg.blockDim = dim3(OneCta<float>::kThreads);
       cfg.dynamicSmemBytes = smem;
       cfg.stream = stream;
       cfg.attrs = &attr;
       cfg.numAttrs = 1;
       e = cudaLaunchKernelExC(&cfg, fn.cluster, args);
     } else if (b.nrounds > 1 && n > 1) {
-      e = cudaLaunchCooperativeKernel(fn.wide, dim3((unsigned)n), dim3(kLockThreads), args, smem, stream);
+      e = cudaLaunchCooperativeKernel(wide, dim3((unsigned)n), block, args, smem, stream);
     } else {
-      e = cudaLaunchKernel(fn.wide, dim3((unsigned)n), dim3(kLockThreads), args, smem, stream);
+      e = cudaLaunchKernel(wide, dim3((unsigned)n), block, args, smem, stream);
     }
   }
   if (e != cudaSuccess) {

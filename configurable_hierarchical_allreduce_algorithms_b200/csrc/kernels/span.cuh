@@ -125,8 +125,6 @@ __device__ __forceinline__ uint4 funnel16(const uint4& lo, const uint4& hi, unsi
   return make_uint4(__funnelshift_r(w0, w1, b), __funnelshift_r(w1, w2, b), __funnelshift_r(w2, w3, b), __funnelshift_r(w3, w4, b));
 }
 
-template <typename T> constexpr int kUnroll16 = Elem<T>::kPerVec > 8 ? 1 : 2;   // (16 accumulators a vector for bytes)
-
 // 128-bit loop for pointers that do not share an alignment.  Vector j covers bytes [pos + 16 j, +16) of every pointer;
 // dst[.] + pos is 16-byte aligned, sources need not be.  The caller guarantees that the two aligned words around each
 // vector lie inside the source.  A warp takes 32 * U consecutive vectors, so that all but its last word are shared.
@@ -250,8 +248,8 @@ __device__ __forceinline__ void copy_loop16(const char* src, char* const* dst, i
 // in shared memory; the destinations are equal modulo 16 (the caller issues one span for each otherwise).
 // A source may be a destination as well (same address, same element): every element is loaded by the thread that
 // stores it, also in the shifted loop, where such a source lies on the destination's grid and needs no shift.
-// G1, G2 / U2: sources (and vectors) in flight in the 256-bit loop for short and for long spans.
-template <typename T, int G1, int G2, int U2>
+// Shape: what is in flight per thread, see below.
+template <typename T, typename Shape>
 __device__ __forceinline__ void reduce_span(const char* const* src, int nsrc, char* const* dst, int ndst, long long count,
                                             int op, bool plain, bool do_scale, float scale) {
   using Acc = typename Elem<T>::Acc;
@@ -268,10 +266,10 @@ __device__ __forceinline__ void reduce_span(const char* const* src, int nsrc, ch
     const int nw = (int)((bytes - lo) / 32);       // (a span is far below 2^31 vectors)
     hi = lo + (long long)nw * 32;
     const int j0 = tid;
-    if (plain) copy_loop32<4>(src[0] + lo, dst, ndst, lo, j0, nw, nt);
+    if (plain) copy_loop32<Shape::kCopy32>(src[0] + lo, dst, ndst, lo, j0, nw, nt);
     else if (op != OP_SUM) reduce_loop32<T, false, 2, 1>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
-    else if (nw <= nt) reduce_loop32<T, true, G1, 1>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
-    else reduce_loop32<T, true, G2, U2>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
+    else if (Shape::kUnroll == 1 || nw <= nt) reduce_loop32<T, true, Shape::kShort, 1>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
+    else reduce_loop32<T, true, Shape::kLong, Shape::kUnroll>(src, lo, nsrc, dst, ndst, lo, j0, nw, nt, op, do_scale, scale);
   } else {
     lo = (long long)((16ull - (d0 & 15ull)) & 15ull);
     long long room = 0;                      // bytes that have to follow the last vector
@@ -280,8 +278,8 @@ __device__ __forceinline__ void reduce_span(const char* const* src, int nsrc, ch
     const long long left = bytes - lo - room;
     const long long nv = left > 0 ? left / 16 : 0;
     hi = lo + nv * 16;
-    if (plain) copy_loop16<4>(src[0], dst, ndst, lo, nv);
-    else if (op == OP_SUM) reduce_loop16<T, true, 2, kUnroll16<T>>(src, nsrc, dst, ndst, lo, nv, op, do_scale, scale);
+    if (plain) copy_loop16<Shape::kCopy16>(src[0], dst, ndst, lo, nv);
+    else if (op == OP_SUM) reduce_loop16<T, true, 2, Shape::kUnroll16>(src, nsrc, dst, ndst, lo, nv, op, do_scale, scale);
     else reduce_loop16<T, false, 2, 1>(src, nsrc, dst, ndst, lo, nv, op, do_scale, scale);
   }
   // both ends, element by element (by the last threads: in a short span they had no vector and start at once)
@@ -309,12 +307,22 @@ struct SpanArgs {
   int op, plain, do_scale;   // plain: one source and no scale
   float scale;
 };
-template <typename T>
+// Loads in flight.  A span with at most one vector per thread is bound by the depth of its chain of round trips: several
+// sources at a time; longer ones by bytes in flight: fewer sources, two vectors deep.
+// OneCta: 128 registers a thread (512 threads, one CTA an SM): 128 bytes a thread, 64 KiB an SM.
+template <typename T> struct OneCta {
+  static constexpr int kThreads = 512, kPerSm = 1;
+  static constexpr bool kWide = sizeof(T) > 1;                     // (16 accumulators a vector for bytes)
+  static constexpr int kShort = kWide ? 4 : 2, kLong = 2, kUnroll = kWide ? 2 : 1, kUnroll16 = kWide ? 2 : 1, kCopy32 = 4, kCopy16 = 4;
+};
+// TwoCtas: 80 registers (384 threads, two CTAs an SM): one vector of as many sources as fit, up to 96 KiB an SM.
+template <typename T> struct TwoCtas {
+  static constexpr int kThreads = 384, kPerSm = 2;
+  static constexpr int kShort = sizeof(T) > 2 ? 4 : 2, kLong = 2, kUnroll = 1, kUnroll16 = 1, kCopy32 = 3, kCopy16 = 3;
+};
+template <typename T, typename Shape>
 __device__ __forceinline__ void run_span(const SpanArgs* a) {
-  constexpr bool wide = sizeof(T) > 1;
-  // a span with at most one vector per thread is bound by the depth of its chain of round trips: four sources at a
-  // time; longer ones by bytes in flight: two sources, two vectors deep (the same 128 bytes per thread)
-  reduce_span<T, wide ? 4 : 2, 2, wide ? 2 : 1>(a->src, a->nsrc, a->dst, a->ndst, a->count, a->op, a->plain != 0, a->do_scale != 0, a->scale);
+  reduce_span<T, Shape>(a->src, a->nsrc, a->dst, a->ndst, a->count, a->op, a->plain != 0, a->do_scale != 0, a->scale);
 }
 
 }  // namespace chb

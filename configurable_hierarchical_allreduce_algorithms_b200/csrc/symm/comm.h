@@ -43,9 +43,9 @@ struct chb_comm {
   // flagged-line form of compiled programs: key = program id * 16 + element size; value = device tables
   // and the line count of the busiest level (sizes the grid)
   std::map<uint64_t, std::pair<void*, std::pair<long long, long long>>> ll_blobs;   // blob, (busiest level lines, largest rank table bytes)
-  // lockstep form of compiled programs (emulated worlds), by 2 * program id + rewriting: grains of the busiest round, element loads and
+  // lockstep form of compiled programs (emulated worlds), by 2 * program id + rewriting: grains and cost of the busiest round, element loads and
   // stores in all, the bits set in any offset or length
-  struct LockBlob { void* dev = nullptr; int bytes = 0, nrefs = 0, nrounds = 0, saved_rounds = 0; long long max_grains = 0, accesses = 0, grid = 0; };
+  struct LockBlob { void* dev = nullptr; int bytes = 0, nrefs = 0, nrounds = 0, saved_rounds = 0; long long max_grains = 0, max_cost = 0, accesses = 0, grid = 0; };
   std::map<uint64_t, LockBlob> lock_blobs;
   std::string last_error;
   // set only by the native constructors (chb_comm_create_ipc / chb_comm_create_emulated), which own the heap
