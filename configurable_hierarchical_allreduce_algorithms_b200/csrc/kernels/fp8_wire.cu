@@ -241,6 +241,168 @@ fp8_rs_kernel(World w, Fp8Io io, long long n, float out_scale) {
   rank_exit(c, nct, [&](Ctrl* cc) { cc->bar_seq = seq + 2ull; });
 }
 
+// ------------------------------------------------------------------ all ranks on one GPU
+// With every rank's input at hand nothing has to cross a wire: a group is quantised and dequantised in registers, with
+// the arithmetic of the kernel above operation for operation (the results are its bits), so the 2 x 7/8 of a byte an
+// element that the wire buffer costs (written, read back) and the barriers between its two phases fall away.
+// What bounds it: HBM for the inputs, closely followed by instruction issue (6 - 7 an element: unpack, scale, convert to
+// e4m3 and back, multiply-add).  The split: a lane holds 32 bytes of a group, so the 128 elements of a group are 8 lanes
+// (16 for fp32) and its largest magnitude takes 3 (4) shuffles for 16 (8) elements, on packed pairs for bf16; kFuseBatch
+// sources are in flight per lane.
+// Measured on one B200, 8 ranks x 64 MiB of bf16: 268 us through the wire buffer -> 124 us (604 MB in and out: 4.9 TB/s).
+constexpr int kFuseThreads = 256;
+constexpr int kFuseBatch = 4;
+
+template <typename T> struct Lane32;      // 32 bytes of a group in one lane
+template <> struct Lane32<float> {
+  static constexpr int kElems = 8, kLanes = 16;
+  static __device__ __forceinline__ void unpack(const uint4& lo, const uint4& hi, float* x) {
+    const float* a = reinterpret_cast<const float*>(&lo);
+    const float* b = reinterpret_cast<const float*>(&hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { x[i] = a[i]; x[4 + i] = b[i]; }
+  }
+  static __device__ __forceinline__ float amax(const uint4& lo, const uint4& hi) {
+    float x[8], m = 0.f;
+    unpack(lo, hi, x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(x[i]));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+  }
+  static __device__ __forceinline__ void store(float* p, const float* x) {
+    uint4 lo, hi;
+    float* a = reinterpret_cast<float*>(&lo);
+    float* b = reinterpret_cast<float*>(&hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { a[i] = x[i]; b[i] = x[4 + i]; }
+    st16(p, lo);
+    st16(p + 4, hi);
+  }
+};
+template <> struct Lane32<__nv_bfloat16> {
+  static constexpr int kElems = 16, kLanes = 8;
+  static __device__ __forceinline__ void unpack(const uint4& lo, const uint4& hi, float* x) {
+    const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&lo);
+    const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(a[i]), g = __bfloat1622float2(b[i]);
+      x[2 * i] = f.x; x[2 * i + 1] = f.y; x[8 + 2 * i] = g.x; x[8 + 2 * i + 1] = g.y;
+    }
+  }
+  static __device__ __forceinline__ float amax(const uint4& lo, const uint4& hi) {
+    const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(&lo);
+    const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&hi);
+    __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m = __hmax2(m, __hmax2(__habs2(a[i]), __habs2(b[i])));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) m = __hmax2(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float2 f = __bfloat1622float2(m);
+    return fmaxf(f.x, f.y);
+  }
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float* x) {
+    uint4 lo, hi;
+    __nv_bfloat162* a = reinterpret_cast<__nv_bfloat162*>(&lo);
+    __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[i] = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+      b[i] = __floats2bfloat162_rn(x[8 + 2 * i], x[8 + 2 * i + 1]);
+    }
+    st16(p, lo);
+    st16(p + 8, hi);
+  }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kFuseThreads, 4)
+fp8_rs_local_kernel(World w, Fp8Io io, long long n, float out_scale) {
+  using L = Lane32<T>;
+  constexpr int E = L::kElems, GW = 32 / L::kLanes;          // elements a lane, groups a warp
+  __shared__ int s_ok;
+  const int P = w.P;
+  if (threadIdx.x == 0) s_ok = 1;
+  __syncthreads();
+  if ((int)threadIdx.x < P && ld_volatile_u32(&w.ctrl[threadIdx.x]->abort)) s_ok = 0;
+  __syncthreads();
+  const long long gpb = n / kGroup, tiles = (gpb + GW - 1) / GW;      // a tile: the groups one warp takes at once
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = ((long long)gridDim.x * kFuseThreads) >> 5;
+  const long long total = s_ok ? tiles * P : 0;
+  for (long long t = ((long long)blockIdx.x * kFuseThreads + threadIdx.x) >> 5; t < total; t += nwarps) {   // uniform per warp
+    const int rank = (int)(t / tiles);
+    const long long g = (t - rank * tiles) * GW + lane / L::kLanes;
+    const bool live = g < gpb;
+    const long long at = live ? g * kGroup + (lane % L::kLanes) * E : 0;      // element of the block
+    const long long from = (long long)rank * n + at;
+    float acc[E];
+    {
+      uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+      if (live) { const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(io.in[rank]) + from); lo = __ldcg(p); hi = __ldcg(p + 1); }
+      float x[E];
+      L::unpack(lo, hi, x);
+#pragma unroll
+      for (int i = 0; i < E; ++i) acc[i] = 0.f + x[i];       // its own block never goes through fp8
+    }
+#pragma unroll 1
+    for (int j0 = 0; j0 < P - 1; j0 += kFuseBatch) {
+      uint4 v[kFuseBatch][2];
+#pragma unroll
+      for (int jj = 0; jj < kFuseBatch; ++jj) {
+        v[jj][0] = v[jj][1] = make_uint4(0u, 0u, 0u, 0u);
+        if (live && j0 + jj < P - 1) {
+          int q = rank + 1 + j0 + jj;
+          if (q >= P) q -= P;
+          const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(io.in[q]) + from);
+          v[jj][0] = __ldcg(p);
+          v[jj][1] = __ldcg(p + 1);
+        }
+      }
+#pragma unroll
+      for (int jj = 0; jj < kFuseBatch; ++jj) {
+        if (j0 + jj >= P - 1) break;                          // uniform
+        const float amax = L::amax(v[jj][0], v[jj][1]);
+        const float sc = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
+        const float inv = 1.0f / sc;
+        float x[E];
+        L::unpack(v[jj][0], v[jj][1], x);
+#pragma unroll
+        for (int i = 0; i < E / 2; ++i) {
+          const float2 d = fp8x2_to_float2(__nv_cvt_float2_to_fp8x2(make_float2(x[2 * i] * inv, x[2 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3));
+          acc[2 * i] += d.x * sc;
+          acc[2 * i + 1] += d.y * sc;
+        }
+      }
+    }
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) acc[i] *= out_scale;
+      L::store(reinterpret_cast<T*>(io.out[rank]) + at, acc);
+    }
+  }
+  rank_exit(w.ctrl[0], gridDim.x, [&](Ctrl*) {
+    for (int r = 1; r < w.P; ++r) w.ctrl[r]->status[6] += 1ull;      // (rank_exit counts rank 0's launch)
+  });
+}
+
+// All ranks here, no per-rank stamps wanted, and no output on top of an input other than the rank's own block in place.
+static bool fp8_local_ok(const chb_comm* c, const void* const* in, void* const* out, size_t block) {
+  if (c->nlocal != c->P || c->P < 2 || c->trace) return false;
+  for (int b = 0; b < c->P; ++b) {
+    const char* o = (const char*)out[b];
+    for (int a = 0; a < c->P; ++a) {
+      const char* i = (const char*)in[a];
+      if (o < i + block * (size_t)c->P && i < o + block && !(a == b && o == i + block * (size_t)a)) return false;
+      const char* q = (const char*)out[a];
+      if (a != b && q < o + block && o < q + block) return false;
+    }
+  }
+  return true;
+}
+
 }  // namespace chb
 
 using namespace chb;
@@ -264,6 +426,16 @@ int chb_rs_fp8_wire(chb_comm* c, int dtype, const void* const* in, void* const* 
     io.out[c->rank + l] = (char*)out[l];
   }
   if (n == 0) return CHB_SUCCESS;
+  if (fp8_local_ok(c, in, out, (size_t)n * (size_t)dtype_size(dtype))) {
+    const long long warps = (long long)c->P * ((n / kGroup + 3) / 4);
+    long long ctas = (warps * 32 + kFuseThreads - 1) / kFuseThreads;
+    const long long most = nctas > 0 ? (long long)nctas * c->P : (long long)c->sm_count * 4;      // resident at once
+    if (ctas > most) ctas = most;
+    if (dtype == DT_F32) fp8_rs_local_kernel<float><<<(unsigned)ctas, kFuseThreads, 0, stream>>>(c->world, io, n, out_scale);
+    else fp8_rs_local_kernel<__nv_bfloat16><<<(unsigned)ctas, kFuseThreads, 0, stream>>>(c->world, io, n, out_scale);
+    if (cudaGetLastError() != cudaSuccess) { c->last_error = "fp8 reduce-scatter launch failed"; return CHB_ERR_CUDA; }
+    return CHB_SUCCESS;
+  }
   const int max_pair_ctas = (kSigSlots - kSigNvlsBase) / kMaxRanks;
   int budget = c->max_ctas / c->nlocal;
   if (nctas <= 0) nctas = (int)(((long long)c->P * n / kGroup + 127) / 128);   // about four half-warp iterations per CTA
