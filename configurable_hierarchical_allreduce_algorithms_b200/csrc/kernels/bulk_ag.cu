@@ -163,9 +163,70 @@ ag_bulk_kernel(World w, BulkIo io, long long nbytes) {
   rank_exit(c, gridDim.x, [&](Ctrl* cc) { cc->bar_seq = seq + 2ull; });
 }
 
+// All ranks on one GPU (one launch serves every rank): a piece of a block is read once and stored to all P outputs, instead
+// of being fetched by every rank for itself, and the launch needs no barrier (its inputs are final in stream order and
+// nobody else writes).
+// Bound by HBM writes: P - 1 of P bytes moved are stores.  Plain vector stores from many short CTAs, four vectors a thread
+// (one piece of 32 KiB a CTA, all CTAs in one moving window of every output); a ring of bulk copies, one stage stored P
+// times by one thread an SM, ran at 115 us where this takes 94.
+// Measured on one B200, 8 ranks, 8 MiB of bf16 a rank: 166 us fetching P times -> 94 us (604 MB in and out: 6.4 TB/s).
+constexpr int kLocalThreads = 256, kLocalUnroll = 4;
+
+// WIDE: 32-byte vectors (every pointer and the block length a multiple of 32), else 16-byte ones.
+template <bool WIDE>
+__global__ void __launch_bounds__(kLocalThreads)
+ag_local_kernel(World w, BulkIo io, long long nbytes) {
+  constexpr int V = WIDE ? 32 : 16;
+  const int P = w.P, owner = (int)blockIdx.y;
+  const unsigned aborted = (int)threadIdx.x < P ? ld_volatile_u32(&w.ctrl[threadIdx.x]->abort) : 0u;   // (travels with the data)
+  const long long nv = nbytes / V, j0 = (long long)blockIdx.x * (kLocalThreads * kLocalUnroll) + threadIdx.x;
+  const char* src = io.in[owner];
+  uint4 lo[kLocalUnroll], hi[kLocalUnroll];
+#pragma unroll
+  for (int u = 0; u < kLocalUnroll; ++u) {
+    const long long j = j0 + u * kLocalThreads;
+    lo[u] = hi[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (j < nv) {
+      if (WIDE) ld32_cg(src + j * V, lo[u], hi[u]);
+      else lo[u] = ld16_cg(src + j * V);
+    }
+  }
+  if (__syncthreads_or((int)aborted)) return;
+  for (int i = 0; i < P; ++i) {
+    char* dst = io.out[i] + (long long)owner * nbytes;
+    if (dst == src) continue;                      // (a block that already lies in its slot)
+#pragma unroll
+    for (int u = 0; u < kLocalUnroll; ++u) {
+      const long long j = j0 + u * kLocalThreads;
+      if (j < nv) {
+        if (WIDE) st32(dst + j * V, lo[u], hi[u]);
+        else st16(dst + j * V, lo[u]);
+      }
+    }
+  }
+  // (no wait can expire here, so the launch counters need no order with the copies)
+  if (blockIdx.x == 0 && owner == 0 && (int)threadIdx.x < P) w.ctrl[threadIdx.x]->status[6] += 1ull;
+}
+
 }  // namespace chb
 
 using namespace chb;
+
+// All ranks here, no per-rank stamps wanted, and no output on top of an input except a block that already lies in its slot.
+static bool bulk_local_ok(const chb_comm* c, const void* const* in, void* const* out, long long nbytes) {
+  if (c->nlocal != c->P || c->P < 2 || c->trace) return false;
+  const size_t ni = (size_t)nbytes, no = ni * (size_t)c->P;
+  for (int b = 0; b < c->P; ++b) {
+    const char* o = (const char*)out[b];
+    for (int a = 0; a < c->P; ++a) {
+      const char* i = (const char*)in[a];
+      if (i < o + no && o < i + ni && !(a == b && i == o + ni * (size_t)a)) return false;
+      const char* q = (const char*)out[a];
+      if (a != b && q < o + no && o < q + no) return false;
+    }
+  }
+  return true;
+}
 
 extern "C" {
 
@@ -194,6 +255,17 @@ int chb_ag_bulk(chb_comm* c, const void* const* in, void* const* out, long long 
     }
   }
   if (nbytes == 0) return CHB_SUCCESS;
+  if (bulk_local_ok(c, in, out, nbytes)) {
+    unsigned long long low = (unsigned long long)nbytes;
+    for (int l = 0; l < c->P; ++l) low |= (unsigned long long)(uintptr_t)in[l] | (unsigned long long)(uintptr_t)out[l];
+    const bool wide = (low & 31ull) == 0ull;
+    const long long piece = (long long)kLocalThreads * kLocalUnroll * (wide ? 32 : 16);
+    const dim3 grid((unsigned)((nbytes + piece - 1) / piece), (unsigned)c->P, 1);
+    if (wide) ag_local_kernel<true><<<grid, kLocalThreads, 0, stream>>>(c->world, io, nbytes);
+    else ag_local_kernel<false><<<grid, kLocalThreads, 0, stream>>>(c->world, io, nbytes);
+    if (cudaGetLastError() != cudaSuccess) { c->last_error = "bulk allgather launch failed"; return CHB_ERR_CUDA; }
+    return CHB_SUCCESS;
+  }
   const int max_pair_ctas = (kSigSlots - kSigNvlsBase) / kMaxRanks;
   int budget = c->max_ctas / c->nlocal;           // 128 KiB of shared memory: one CTA per SM
   static bool attr_set[64] = {};
