@@ -105,28 +105,80 @@ rs_adam_kernel(World w, AdamIo io, long long n, AdamHyper h, const char* mc_grad
   rank_exit(c, gridDim.x, [&](Ctrl* cc) { cc->bar_seq = seq + 2ull; });
 }
 
-// Plain (unsharded) variant for the data-parallel path: the gradient has
-// already been allreduced; AdamW on the fp32 master, bf16 copy of the result.
-__global__ void __launch_bounds__(kAdamThreads)
-adam_flat_kernel(const float* __restrict__ grad, float* master, float* m, float* v, __nv_bfloat16* param,
-                 long long n, AdamHyper h) {
-  const long long nvec = n / 4;
-  const long long TT = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += TT) {
-    const float4 g = reinterpret_cast<const float4*>(grad)[i];
-    float4 ww = reinterpret_cast<float4*>(master)[i], m1 = reinterpret_cast<float4*>(m)[i],
-           v1 = reinterpret_cast<float4*>(v)[i];
+// All ranks on this GPU (P emulated ranks, or a world of one): the gradients are final in stream order, so nobody waits for
+// anybody, and the shards need no persistent CTAs that meet at barriers.
+// Bound by HBM: 4 P + 26 bytes an element of a shard.  One vector of four elements a thread, all P gradient loads (in
+// batches of eight) and the three state loads issued before the first addition, short CTAs.
+// Measured on one B200, 8 ranks x 2 Mi elements a shard: 235 us with barriers and 18 CTAs a rank, 199 us so (each with the allgather
+// of the parameters, 1.2 GB in all).
+constexpr int kLocalAdamThreads = 256;
+
+__global__ void __launch_bounds__(kLocalAdamThreads, 4)
+rs_adam_local_kernel(World w, AdamIo io, long long n, AdamHyper h) {
+  const int P = w.P, rank = (int)blockIdx.y;
+  const unsigned aborted = (int)threadIdx.x < P ? ld_volatile_u32(&w.ctrl[threadIdx.x]->abort) : 0u;   // (travels with the data)
+  const long long nvec = n / 4, i = (long long)blockIdx.x * kLocalAdamThreads + threadIdx.x;
+  const bool live = i < nvec;
+  const long long at = (long long)rank * nvec + i;
+  float4 ww = make_float4(0.f, 0.f, 0.f, 0.f), m1 = ww, v1 = ww, g = ww;
+  if (live) {
+    ww = reinterpret_cast<const float4*>(io.master[rank])[i];
+    m1 = reinterpret_cast<const float4*>(io.m[rank])[i];
+    v1 = reinterpret_cast<const float4*>(io.v[rank])[i];
+  }
+  constexpr int G = 8;
+#pragma unroll 1
+  for (int q0 = 0; q0 < P; q0 += G) {
+    uint4 t[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      t[q] = make_uint4(0u, 0u, 0u, 0u);
+      if (live && q0 + q < P) t[q] = ld16_cg(reinterpret_cast<const char*>(io.grad[q0 + q]) + at * 16);
+    }
+#pragma unroll
+    for (int q = 0; q < G; ++q) {      // rank order: identical bits on every run
+      if (q0 + q < P) {
+        const float4 x = *reinterpret_cast<const float4*>(&t[q]);
+        g.x += x.x; g.y += x.y; g.z += x.z; g.w += x.w;
+      }
+    }
+  }
+  if (__syncthreads_or((int)aborted)) return;
+  if (live) {
     const float s = h.grad_scale;
     __nv_bfloat16 o[4];
     o[0] = __float2bfloat16_rn(adam_one(g.x * s, ww.x, m1.x, v1.x, h));
     o[1] = __float2bfloat16_rn(adam_one(g.y * s, ww.y, m1.y, v1.y, h));
     o[2] = __float2bfloat16_rn(adam_one(g.z * s, ww.z, m1.z, v1.z, h));
     o[3] = __float2bfloat16_rn(adam_one(g.w * s, ww.w, m1.w, v1.w, h));
-    reinterpret_cast<float4*>(master)[i] = ww;
-    reinterpret_cast<float4*>(m)[i] = m1;
-    reinterpret_cast<float4*>(v)[i] = v1;
-    reinterpret_cast<uint2*>(param)[i] = *reinterpret_cast<uint2*>(o);
+    reinterpret_cast<float4*>(io.master[rank])[i] = ww;
+    reinterpret_cast<float4*>(io.m[rank])[i] = m1;
+    reinterpret_cast<float4*>(io.v[rank])[i] = v1;
+    reinterpret_cast<uint2*>(io.param[rank])[i] = *reinterpret_cast<uint2*>(o);
   }
+  if (blockIdx.x == 0 && rank == 0 && (int)threadIdx.x < P) w.ctrl[threadIdx.x]->status[6] += 1ull;
+}
+
+// Plain (unsharded) variant for the data-parallel path: the gradient has
+// already been allreduced; AdamW on the fp32 master, bf16 copy of the result.
+// Bound by HBM (30 bytes an element); one vector a thread, short CTAs, as above.
+__global__ void __launch_bounds__(kLocalAdamThreads)
+adam_flat_kernel(const float* __restrict__ grad, float* master, float* m, float* v, __nv_bfloat16* param,
+                 long long n, AdamHyper h) {
+  const long long i = (long long)blockIdx.x * kLocalAdamThreads + threadIdx.x;
+  if (i >= n / 4) return;
+  const float4 g = reinterpret_cast<const float4*>(grad)[i];
+  float4 ww = reinterpret_cast<float4*>(master)[i], m1 = reinterpret_cast<float4*>(m)[i], v1 = reinterpret_cast<float4*>(v)[i];
+  const float s = h.grad_scale;
+  __nv_bfloat16 o[4];
+  o[0] = __float2bfloat16_rn(adam_one(g.x * s, ww.x, m1.x, v1.x, h));
+  o[1] = __float2bfloat16_rn(adam_one(g.y * s, ww.y, m1.y, v1.y, h));
+  o[2] = __float2bfloat16_rn(adam_one(g.z * s, ww.z, m1.z, v1.z, h));
+  o[3] = __float2bfloat16_rn(adam_one(g.w * s, ww.w, m1.w, v1.w, h));
+  reinterpret_cast<float4*>(master)[i] = ww;
+  reinterpret_cast<float4*>(m)[i] = m1;
+  reinterpret_cast<float4*>(v)[i] = v1;
+  reinterpret_cast<uint2*>(param)[i] = *reinterpret_cast<uint2*>(o);
 }
 
 }  // namespace chb
@@ -174,6 +226,12 @@ int chb_rs_adam(chb_comm* c, const void* const* grad, void* const* master, void*
   }
   if (n == 0) return CHB_SUCCESS;
   AdamHyper h{hyper[0], hyper[1], hyper[2], hyper[3], hyper[4], hyper[5], hyper[6], hyper[7]};
+  if (c->nlocal == c->P && !c->trace && !mc) {
+    const dim3 grid((unsigned)((n / 4 + kLocalAdamThreads - 1) / kLocalAdamThreads), (unsigned)c->P, 1);
+    rs_adam_local_kernel<<<grid, kLocalAdamThreads, 0, stream>>>(c->world, io, n, h);
+    if (cudaGetLastError() != cudaSuccess) { c->last_error = "rs_adam launch failed"; return CHB_ERR_CUDA; }
+    return CHB_SUCCESS;
+  }
   const int max_pair_ctas = (kSigSlots - kSigNvlsBase) / kMaxRanks;
   int budget = c->max_ctas / c->nlocal;
   if (nctas <= 0) nctas = (int)((n / 4 + kAdamThreads * 4 - 1) / (kAdamThreads * 4));
@@ -197,9 +255,8 @@ int chb_adam_flat(const void* grad, void* master, void* m, void* v, void* param_
   if (((uintptr_t)grad | (uintptr_t)master | (uintptr_t)m | (uintptr_t)v) & 15u || ((uintptr_t)param_bf16 & 7u)) return CHB_ERR_ARG;
   if (n == 0) return CHB_SUCCESS;
   AdamHyper h{hyper[0], hyper[1], hyper[2], hyper[3], hyper[4], hyper[5], hyper[6], hyper[7]};
-  long long blocks = (n / 4 + kAdamThreads - 1) / kAdamThreads;
-  if (blocks > 148 * 4) blocks = 148 * 4;
-  adam_flat_kernel<<<(unsigned)blocks, kAdamThreads, 0, stream>>>((const float*)grad, (float*)master, (float*)m, (float*)v,
+  const long long blocks = (n / 4 + kLocalAdamThreads - 1) / kLocalAdamThreads;
+  adam_flat_kernel<<<(unsigned)blocks, kLocalAdamThreads, 0, stream>>>((const float*)grad, (float*)master, (float*)m, (float*)v,
                                                                    (__nv_bfloat16*)param_bf16, n, h);
   return cudaGetLastError() == cudaSuccess ? CHB_SUCCESS : CHB_ERR_CUDA;
 }
