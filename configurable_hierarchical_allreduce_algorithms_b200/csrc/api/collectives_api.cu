@@ -25,6 +25,7 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
                              void* const* out, float scale, int nctas, cudaStream_t stream);
 int chb_lockstep_ok(const chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out,
                     long long slot_bytes);
+int chb_program_fits(const chb_comm* c, const chb_program* p, int dtype);
 int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, long long payload_bytes);
 long long chb_program_ll_lines(const chb_program* p, int esz);
 int chb_ll_collective(chb_comm* c, int mode, int dtype, int op, const void* const* in, void* const* out,
@@ -222,6 +223,12 @@ int chb_collective(chb_comm* c, int coll, const char* algo, int k, int b, int au
   if (rc) return rc;
   if (mode == 0 && chb_lockstep_ok(c, p, dtype, in, out, slot))
     return chb_run_program_lockstep(c, p, dtype, op, in, out, scale, nctas, stream);
+  // Pulled by the interpreter: emulated ranks see each other's caller buffers, registered or not, so nothing is staged (the
+  // program of the general lowering decides what is refused).
+  if (ll_kind && flags < 3 && chb_lockstep_ok(c, p, dtype, in, out, slot) && chb_program_fits(c, p, dtype)) {
+    rc = get_program(c, coll, algo, k, b, aux, count, 3, &p);
+    if (rc) return rc;
+  }
   return chb_run_program(c, p, dtype, op, in, out, scale, nctas, stream);
 }
 

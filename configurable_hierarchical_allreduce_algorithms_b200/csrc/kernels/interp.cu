@@ -26,7 +26,7 @@
 
 namespace chb {
 
-constexpr int kInterpThreads = 512;
+constexpr long long kSpreadBytes = 4 << 20;       // emulated ranks: longer vectors use the CTAs of four an SM
 constexpr long long kSmallStepElems = 16 << 10;  // steps below this many elements are run whole, by one CTA
 
 struct DevStep { long long dst_off; long long count; int dst_buf; int nsrc; int src_begin; unsigned flags; };
@@ -316,8 +316,13 @@ __device__ __forceinline__ void walk_round(const DevRound& R, unsigned nct, Roun
   k->nitems = (long long)k->nsmall + rows * R.nbig;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kInterpThreads, 1)
+// Shape: OneCta for one rank per GPU; emulated ranks share the GPU, and FourCtas spreads each of them over four times as
+// many SMs, so that the two to four ranks which a round of a hierarchical schedule keeps busy reach the whole chip
+// (8 ranks, pulled allreduce of 64 MiB fp32, k = 2, b = 1: 560 us with 18 CTAs a rank and staging, 236 us with 74 and without;
+// k = 2, b = 4, bf16: 917 and 501 us; six or eight smaller CTAs an SM measured the same).  Up to kSpreadBytes the barriers of
+// more CTAs cost what they give.
+template <typename T, typename Shape>
+__global__ void __launch_bounds__(Shape::kThreads, Shape::kPerSm)
 interp_kernel(World w, const char* __restrict__ blob, IoTable io, int op, float scale, int tables_in_smem) {
   extern __shared__ __align__(16) unsigned char interp_tables[];
   const int rank = w.rank0 + (int)blockIdx.y;
@@ -403,7 +408,7 @@ interp_kernel(World w, const char* __restrict__ blob, IoTable io, int op, float 
         long long cnt = st.count - e0;
         if (v >= s_walk.nsmall && cnt > s_walk.te) cnt = s_walk.te;
         __syncthreads();      // the readers of the previous span's arguments are done
-        if (set_step<T>(st, s_walk.srcs, w, io, rank, e0, cnt, op, scale, &s_span, h->limit)) run_span<T, OneCta<T>>(&s_span);
+        if (set_step<T>(st, s_walk.srcs, w, io, rank, e0, cnt, op, scale, &s_span, h->limit)) run_span<T, Shape>(&s_span);
       }
       ok = rank_barrier(c, nct, gen, w.timeout_ns, rank, t);
       if (!ok) break;
@@ -468,15 +473,17 @@ local_copy_kernel(Ctrl* c, const char* __restrict__ src, char* __restrict__ dst,
 
 typedef void (*InterpFn)(World, const char*, IoTable, int, float, int);
 
-static InterpFn pick_kernel(int dtype) {
+template <typename T>
+static InterpFn interp_of(bool spread) { return spread ? (InterpFn)interp_kernel<T, FourCtas<T>> : (InterpFn)interp_kernel<T, OneCta<T>>; }
+static InterpFn pick_kernel(int dtype, bool spread) {
   switch (dtype) {
-    case DT_F32: return interp_kernel<float>;
-    case DT_BF16: return interp_kernel<__nv_bfloat16>;
-    case DT_F16: return interp_kernel<__half>;
-    case DT_I32: return interp_kernel<int32_t>;
-    case DT_F64: return interp_kernel<double>;
-    case DT_I64: return interp_kernel<int64_t>;
-    case DT_U8: return interp_kernel<uint8_t>;
+    case DT_F32: return interp_of<float>(spread);
+    case DT_BF16: return interp_of<__nv_bfloat16>(spread);
+    case DT_F16: return interp_of<__half>(spread);
+    case DT_I32: return interp_of<int32_t>(spread);
+    case DT_F64: return interp_of<double>(spread);
+    case DT_I64: return interp_of<int64_t>(spread);
+    case DT_U8: return interp_of<uint8_t>(spread);
   }
   return nullptr;
 }
@@ -538,8 +545,7 @@ int chb_run_program(chb_comm* c, const chb_program* p, int dtype, int op, const 
   if (!c || !p || !in || !out) return CHB_ERR_ARG;
   const Program& g = p->prog;
   if (g.P != c->P) { c->last_error = "program was compiled for a different number of ranks"; return CHB_ERR_ARG; }
-  InterpFn fn = pick_kernel(dtype);
-  if (!fn) return CHB_ERR_ARG;
+  if (!pick_kernel(dtype, false)) return CHB_ERR_ARG;
   const size_t esz = (size_t)dtype_size(dtype);
   if ((size_t)g.work_elems * esz > c->scratch_bytes) {
     c->last_error = "program needs more symmetric scratch than the communicator has";
@@ -590,19 +596,22 @@ int chb_run_program(chb_comm* c, const chb_program* p, int dtype, int op, const 
       }
     }
   }
-  int per_rank_budget = c->max_ctas / (c->nlocal > 0 ? c->nlocal : 1);
+  const long long bytes = (long long)std::max(g.in_elems, g.out_elems) * (long long)esz;
+  const bool spread = c->nlocal > 1 && nctas <= 0 && bytes > kSpreadBytes;
+  int per_rank_budget = c->max_ctas * (spread ? FourCtas<float>::kPerSm : 1) / (c->nlocal > 0 ? c->nlocal : 1);
   if (per_rank_budget < 1) per_rank_budget = 1;
   if (nctas <= 0) {
     // enough CTAs to keep NVLink busy for large steps, one for latency-bound programs
-    long long bytes = (long long)std::max(g.in_elems, g.out_elems) * (long long)esz;
     // NVLink wants about 2 MB in flight per GPU (rate x loaded latency) and a thread keeps 128 bytes in flight:
     // bandwidth-bound sizes take (nearly) every SM, one CTA each
     nctas = bytes <= (64 << 10) ? 1 : (bytes <= (1 << 20) ? 32 : (bytes <= (4 << 20) ? 64 : 128));
     // a single-rank world only copies locally: HBM-bound, wants every SM
     if (c->P == 1 && bytes > (16 << 20)) nctas = per_rank_budget;
+    if (spread) nctas = per_rank_budget;
   }
   if (nctas > per_rank_budget) nctas = per_rank_budget;
-  dim3 grid((unsigned)nctas, (unsigned)c->nlocal, 1), block(kInterpThreads, 1, 1);
+  const InterpFn fn = pick_kernel(dtype, spread);
+  dim3 grid((unsigned)nctas, (unsigned)c->nlocal, 1), block(spread ? FourCtas<float>::kThreads : OneCta<float>::kThreads, 1, 1);
   World w = c->world;
   const char* blobp = (const char*)blob;
   // a rank's own table entries go to shared memory when they fit what every kernel may have without opting in

@@ -363,6 +363,11 @@ static int get_lock_blob(chb_comm* c, const chb_program* p, int dtype, const chb
   return CHB_SUCCESS;
 }
 
+// Does the communicator's scratch hold the program's?
+int chb_program_fits(const chb_comm* c, const chb_program* p, int dtype) {
+  return (size_t)p->prog.work_elems * (size_t)dtype_size(dtype) <= c->scratch_bytes;
+}
+
 // Small schedules of which the rewriting shortens nothing (recursive doubling, recursive halving: every round is an
 // exchange that reduces) run faster with flagged lines, whose rounds have no barrier: 8 ranks, recursive doubling
 // 40 / 130 / 256 / 512 KB 15.3 / 15.5 / 19.5 / 20.7 us in lockstep, 13.9 / 14.0 / 22.2 / 38.7 us with lines.

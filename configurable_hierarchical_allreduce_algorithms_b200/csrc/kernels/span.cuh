@@ -320,6 +320,10 @@ template <typename T> struct TwoCtas {
   static constexpr int kThreads = 384, kPerSm = 2;
   static constexpr int kShort = sizeof(T) > 2 ? 4 : 2, kLong = 2, kUnroll = 1, kUnroll16 = 1, kCopy32 = 3, kCopy16 = 3;
 };
+// FourCtas: the registers of TwoCtas in smaller CTAs (192 threads, four an SM).
+template <typename T> struct FourCtas : TwoCtas<T> {
+  static constexpr int kThreads = 192, kPerSm = 4;
+};
 template <typename T, typename Shape>
 __device__ __forceinline__ void run_span(const SpanArgs* a) {
   reduce_span<T, Shape>(a->src, a->nsrc, a->dst, a->ndst, a->count, a->op, a->plain != 0, a->do_scale != 0, a->scale);

@@ -99,3 +99,28 @@ def test_lockstep_mixes_with_the_per_rank_kernels(cuda):
         assert torch.equal(outs[6], torch.stack(src).sum(0))
     comm.check()
     comm.close()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_pull_with_many_small_ctas(cuda, dtype):
+    """Pulled vectors beyond 4 MiB spread an emulated rank over four CTAs an SM: same bits as with a given number of
+    large ones, on aligned and odd lengths, private (nothing is staged) and registered buffers."""
+    P = 4
+    comm = Communicator.emulated(P, scratch_bytes=64 << 20, user_bytes=32 << 20)
+    for n in ((5 << 20) // dtype.itemsize, (5 << 20) // dtype.itemsize + 4):      # the second one: slices off the grid
+        src = [torch.randn(n, device="cuda").to(dtype) for _ in range(P)]
+        reg = comm.empty(n, dtype)
+        for x, y in zip(reg, src):
+            x.copy_(y)
+        for k, b in ((2, 1), (2, 2)):
+            want = chb.all_reduce(comm, src, algo="radix_batch:pull", k=k, b=b, nctas=7)
+            for ins in (src, reg):
+                got = chb.all_reduce(comm, ins, algo="radix_batch:pull", k=k, b=b)
+                assert all(torch.equal(x, y) for x, y in zip(got, want)), (n, k, b)
+    comm.check()
+    comm.close()
+    # the scratch that the general lowering asks for is asked for here as well
+    small = Communicator.emulated(P, scratch_bytes=1 << 20, user_bytes=4096)
+    with pytest.raises(chb.CollectiveError):
+        chb.all_reduce(small, [torch.zeros(1 << 20, device="cuda") for _ in range(P)], algo="radix_batch:pull", k=2, b=2)
+    small.close()
