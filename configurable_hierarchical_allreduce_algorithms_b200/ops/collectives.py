@@ -24,6 +24,8 @@ from __future__ import annotations
 import torch
 
 import ctypes as C
+import os
+from functools import lru_cache
 
 from ..parallel.comm import Communicator, CollectiveError, DTYPES, OPS, _stream_ptr
 from ..parallel.program import ProgramError
@@ -51,6 +53,11 @@ def _ll_ok(comm, ins, outs, payload_bytes):
     return all((t.data_ptr() % 8) == 0 for t in ins + outs)
 
 
+@lru_cache(maxsize=None)
+def _ptr_array(n: int):
+    return C.c_void_p * n
+
+
 # kernels and programs that take an allreduce of any length; every other schedule cuts the vector into P slices
 _ANY_COUNT = ("ll", "ll2", "nvls", "nvls1", "recursive_doubling", "ring", "k_reduce_scatter_allgather",
               "recursive_multiplying", "recursive_exchange", "inter_reduce_exchange_bcast")
@@ -70,13 +77,39 @@ def any_count(coll: str, algo: str, k: int, b: int, count: int, P: int, ll_ok: b
 
 _COLL = {"allreduce": 0, "reduce_scatter": 1, "allgather": 2, "alltoall": 3, "gather": 4, "phase": 5}
 _ALGO_BYTES: dict = {}
-_NVTX = __import__("os").environ.get("CHB_NVTX", "0") == "1"   # NVTX range around every launch
+_NVTX = os.environ.get("CHB_NVTX", "0") == "1"   # NVTX range around every launch
+
+
+def _run_local(comm: Communicator, coll: str, ins, outs, count: int, op, scale, stream, payload_bytes: int) -> bool:
+    """An emulated world's automatic choice of a flagged-line kernel runs as one lockstep launch with the same result;
+    False: not such a call (nothing was enqueued)."""
+    dtype = ins[0].dtype
+    key = (coll, payload_bytes, dtype)
+    plan = comm._local_plans.get(key, -1)
+    if plan == -1:
+        choice = autotune.choose(comm, coll, payload_bytes, dtype, False)      # (no multicast here: any buffers)
+        plan = None if os.environ.get("CHB_ALGO") else {"ll": 0, "ll2": 1}.get(choice.algo)      # (a pinned kernel stays)
+        comm._local_plans[key] = plan
+    if plan is None or len(ins) != comm.nlocal or len(outs) != comm.nlocal:
+        return False
+    rc = N.lib().chb_collective_local(comm._h, _COLL[coll], plan, DTYPES[dtype], OPS[op],
+                                      comm._pack_ptrs(*[t.data_ptr() for t in ins], *[t.data_ptr() for t in outs]),
+                                      count, scale, _stream_ptr(stream))
+    if rc == N.ERR_UNSUPPORTED:
+        return False
+    if rc:
+        comm._err(rc)
+    comm.launches += 1
+    return True
 
 
 def _run(comm: Communicator, coll: str, ins, outs, count: int, op, algo, k, b, aux, scale, nctas, stream,
          payload_bytes: int, ll_mode: int):
     """Pick the kernel and enqueue it with a single native call."""
     auto = algo == "auto"
+    if auto and comm.nlocal > 1 and nctas == 0 and not _NVTX:
+        if _run_local(comm, coll, ins, outs, count, op, scale, stream, payload_bytes):
+            return
     if auto:
         sym = comm.is_symmetric(ins[0]) and comm.is_symmetric(outs[0])
         key = (coll, payload_bytes, ins[0].dtype, sym)
@@ -94,6 +127,9 @@ def _run(comm: Communicator, coll: str, ins, outs, count: int, op, algo, k, b, a
         elif algo.startswith("nvls") and not (comm.has_multicast and sym and comm.nlocal == 1
                                               and payload_bytes % 16 == 0):
             algo, k, b = "radix_batch", 2, 1
+        if comm.nlocal > 1 and algo.startswith("radix_batch:"):
+            algo = "radix_batch"                # mode and CTAs were measured with one rank per GPU
+            nctas = 0 if nctas == choice.nctas else nctas
         if coll == "allreduce" and count % comm.P:
             algo, k, b = any_count(coll, algo, k, b, count, comm.P, _ll_ok(comm, ins, outs, payload_bytes), payload_bytes)
     if algo == "bulk" and not (coll == "allgather" and payload_bytes % 16 == 0 and comm.is_symmetric(ins[0])
@@ -108,15 +144,15 @@ def _run(comm: Communicator, coll: str, ins, outs, count: int, op, algo, k, b, a
     if _NVTX:
         torch.cuda.nvtx.range_push(f"chb.{coll}.{algo}[{payload_bytes}B]")
     rc = N.lib().chb_collective(comm._h, _COLL[coll], ab, k, b, aux, DTYPES[ins[0].dtype], OPS[op],
-                                (C.c_void_p * n)(*[t.data_ptr() for t in ins]),
-                                (C.c_void_p * n)(*[t.data_ptr() for t in outs]),
+                                _ptr_array(n)(*[t.data_ptr() for t in ins]),
+                                _ptr_array(n)(*[t.data_ptr() for t in outs]),
                                 count, scale, nctas, _stream_ptr(stream))
     if rc == N.ERR_COUNT and auto and algo.endswith(":ll"):
         # the tuned row was measured with a larger flagged-line inbox than this communicator has: same program, pulled
         ab = (algo[:-3] + ":pull").encode()
         rc = N.lib().chb_collective(comm._h, _COLL[coll], ab, k, b, aux, DTYPES[ins[0].dtype], OPS[op],
-                                    (C.c_void_p * n)(*[t.data_ptr() for t in ins]),
-                                    (C.c_void_p * n)(*[t.data_ptr() for t in outs]),
+                                    _ptr_array(n)(*[t.data_ptr() for t in ins]),
+                                    _ptr_array(n)(*[t.data_ptr() for t in outs]),
                                     count, scale, nctas, _stream_ptr(stream))
     if _NVTX:
         torch.cuda.nvtx.range_pop()

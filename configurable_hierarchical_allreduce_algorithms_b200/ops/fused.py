@@ -4,6 +4,8 @@ wire format, and reduce-scatter fused with the sharded AdamW update
 from __future__ import annotations
 
 import ctypes as C
+import struct
+from functools import lru_cache
 
 import torch
 
@@ -16,9 +18,15 @@ N.optional("chb_rs_adam", i32, [vp, C.POINTER(vp), C.POINTER(vp), C.POINTER(vp),
                                 C.c_longlong, C.POINTER(f32), i32, i32, vp])
 
 
-N.optional("chb_adam_flat", i32, [vp, vp, vp, vp, vp, C.c_longlong, C.POINTER(f32), vp])
-N.optional("chb_bucket_fill", i32, [vp, i32, C.POINTER(vp), C.POINTER(C.c_longlong), C.POINTER(C.c_longlong),
-                                    C.POINTER(i32), C.POINTER(C.c_ubyte), vp])
+# (tables travel as packed bytes: building a ctypes array costs several times as much as packing one)
+N.optional("chb_adam_flat", i32, [vp, vp, vp, vp, vp, C.c_longlong, C.c_char_p, vp])
+N.optional("chb_bucket_fill", i32, [vp, i32, C.c_char_p, C.c_char_p, C.c_char_p, C.c_char_p, C.c_char_p, vp])
+_pack_hyper = struct.Struct("8f").pack
+
+
+@lru_cache(maxsize=None)
+def _packers(k: int):
+    return tuple(struct.Struct(f"{k}{c}").pack for c in "Qqi")
 
 
 def bucket_fill(bucket: torch.Tensor, items, stream=None):
@@ -30,12 +38,11 @@ def bucket_fill(bucket: torch.Tensor, items, stream=None):
         return
     assert bucket.dtype == torch.float32 and bucket.is_cuda
     grads = [g if g.is_contiguous() else g.contiguous() for g, _, _ in items]
-    src = (vp * k)(*[g.data_ptr() for g in grads])
-    off = (C.c_longlong * k)(*[int(o) for _, o, _ in items])
-    n = (C.c_longlong * k)(*[g.numel() for g in grads])
-    dt = (i32 * k)(*[DTYPES[g.dtype] for g in grads])
-    ow = (C.c_ubyte * k)(*[1 if w else 0 for _, _, w in items])
-    rc = N.lib().chb_bucket_fill(bucket.data_ptr(), k, src, off, n, dt, ow, _stream_ptr(stream))
+    pack_ptr, pack_len, pack_int = _packers(k)
+    rc = N.lib().chb_bucket_fill(bucket.data_ptr(), k, pack_ptr(*[g.data_ptr() for g in grads]),
+                                 pack_len(*[int(o) for _, o, _ in items]), pack_len(*[g.numel() for g in grads]),
+                                 pack_int(*[DTYPES[g.dtype] for g in grads]), bytes([1 if w else 0 for _, _, w in items]),
+                                 _stream_ptr(stream))
     if rc:
         raise RuntimeError(f"chb_bucket_fill failed with code {rc}")
 
@@ -44,7 +51,7 @@ def adam_flat(grad, master, exp_avg, exp_avg_sq, param_bf16, *, lr, betas=(0.9, 
               step=1, grad_scale=1.0, stream=None):
     """AdamW on a flat fp32 master tensor fed by a flat fp32 gradient; writes the bf16 parameters."""
     n = master.numel()
-    hyper = (f32 * 8)(lr, betas[0], betas[1], eps, weight_decay, 1.0 - betas[0] ** step, 1.0 - betas[1] ** step, grad_scale)
+    hyper = _pack_hyper(lr, betas[0], betas[1], eps, weight_decay, 1.0 - betas[0] ** step, 1.0 - betas[1] ** step, grad_scale)
     rc = N.lib().chb_adam_flat(grad.data_ptr(), master.data_ptr(), exp_avg.data_ptr(), exp_avg_sq.data_ptr(),
                                param_bf16.data_ptr(), n, hyper, _stream_ptr(stream))
     if rc:

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from typing import Sequence
 
 import torch
@@ -53,6 +54,7 @@ N.optional("chb_program_ll_lines", C.c_longlong, [vp, i32])
 N.optional("chb_ll_max_bytes", C.c_longlong, [vp])
 N.optional("chb_ll_collective", i32, [vp, i32, i32, i32, C.POINTER(vp), C.POINTER(vp), C.c_longlong, f32, i32, vp])
 N.optional("chb_collective", i32, [vp, i32, C.c_char_p, i32, i32, i32, i32, i32, C.POINTER(vp), C.POINTER(vp), i64, f32, i32, vp])
+N.optional("chb_collective_local", i32, [vp, i32, i32, i32, i32, C.c_char_p, i64, f32, vp])
 N.optional("chb_bootstrap_create", i32, [C.c_char_p, i32, i32, i32, C.POINTER(vp)])
 N.optional("chb_bootstrap_barrier", i32, [vp])
 N.optional("chb_bootstrap_destroy", None, [vp])
@@ -89,8 +91,9 @@ class _CudaBuf:
 
 
 def _stream_ptr(stream=None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())     # (no Stream object: a tenth of the time)
 
 
 class Communicator:
@@ -109,6 +112,7 @@ class Communicator:
         self._programs = {}
         self._choices = {}       # (collective, bytes, dtype, symmetric) -> autotune.Choice
         self._user_ranges = []
+        self._local_plans = {}   # emulated worlds: (collective, bytes, dtype) -> 0 / 1 (one- / two-shot lines) or None
         self._host_pipelines = {}  # (dtype, chunk, depth) -> ops.host.HostAllReduce
         self.group = None
         return self
@@ -295,6 +299,7 @@ class Communicator:
         self.ll_max_bytes, self.sm_count, self.has_multicast = int(info[8]), int(info[9]), bool(info[10])
         self.ll2_max_bytes = (self.ll_max_bytes // 16) * 8 * P   # two-shot flagged lines: half a slot per slice
         self.set_timeout_us(int(os.environ.get("CHB_TIMEOUT_US", timeout_us)))
+        self._pack_ptrs = struct.Struct(f"{2 * nlocal}Q").pack
         self.launches = 0   # kernels launched by this communicator (all local ranks count as one)
 
     def close(self):

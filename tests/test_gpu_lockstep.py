@@ -124,3 +124,31 @@ def test_pull_with_many_small_ctas(cuda, dtype):
     with pytest.raises(chb.CollectiveError):
         chb.all_reduce(small, [torch.zeros(1 << 20, device="cuda") for _ in range(P)], algo="radix_batch:pull", k=2, b=2)
     small.close()
+
+
+@pytest.mark.parametrize("P", [2, 3, 8])
+def test_automatic_small_calls_equal_the_line_kernels(cuda, P):
+    """`auto` in an emulated world: the bits of the flagged-line kernels, on odd lengths, for every type and operation;
+    in place and on misaligned buffers the line kernels and programs themselves run."""
+    comm = Communicator.emulated(P, ll_bytes=1 << 20, scratch_bytes=8 << 20, user_bytes=4096)
+    g = torch.Generator(device="cuda").manual_seed(P)
+    for dtype in (torch.float32, torch.bfloat16, torch.float16, torch.int32, torch.float64, torch.uint8):
+        for n in (1, 7, 2049, 15001):       # (blocks up to the 128 KiB where every table and rule still picks the lines)
+            src = [torch.rand(n * P, generator=g, device="cuda").mul_(9).to(dtype) for _ in range(P)]
+            for op, scale in (("sum", 1.0), ("sum", 0.5), ("max", 1.0)):
+                whole = [s[:n] for s in src]
+                assert all(torch.equal(a, b) for a, b in zip(chb.all_reduce(comm, whole, op=op, scale=scale),
+                                                             chb.all_reduce(comm, whole, op=op, scale=scale, algo="ll")))
+            got, want = chb.reduce_scatter(comm, src), chb.reduce_scatter(comm, src, algo="ll")
+            assert all(torch.equal(a, b) for a, b in zip(got, want)), (dtype, n)
+            blocks = [s[:n] for s in src]
+            assert all(torch.equal(a, torch.cat(blocks)) for a in chb.all_gather(comm, blocks))
+            bufs = [s[:n].clone() for s in src]
+            chb.all_reduce(comm, bufs, out=bufs)
+            assert all(torch.equal(a, b) for a, b in zip(bufs, chb.all_reduce(comm, blocks, algo="ll"))), (dtype, n)
+    ins = [torch.randn(4097, device="cuda")[1:] for _ in range(P)]
+    full = torch.stack(ins).sum(0)
+    for y in chb.all_reduce(comm, ins):
+        torch.testing.assert_close(y, full, rtol=1e-5, atol=1e-5 * P)
+    comm.check()
+    comm.close()
