@@ -468,7 +468,12 @@ local_copy_kernel(Ctrl* c, const char* __restrict__ src, char* __restrict__ dst,
       if (i < nvec) st32(dst + i * 32, lo[u], hi[u]);
     }
   }
-  rank_exit(c, gridDim.x, [&](Ctrl* cc) { cc->epoch = cc->epoch + (unsigned long long)nrounds; });
+  // (nobody waits in a world of one: the counters need no order with the copies, and a fence at the end of every CTA costs
+  // 1 us of a 20 MiB copy)
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    c->epoch += (unsigned long long)nrounds;
+    c->status[6] += 1ull;
+  }
 }
 
 typedef void (*InterpFn)(World, const char*, IoTable, int, float, int);

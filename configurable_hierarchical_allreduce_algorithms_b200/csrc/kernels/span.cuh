@@ -318,7 +318,7 @@ template <typename T> struct OneCta {
 // TwoCtas: 80 registers (384 threads, two CTAs an SM): one vector of as many sources as fit, up to 96 KiB an SM.
 template <typename T> struct TwoCtas {
   static constexpr int kThreads = 384, kPerSm = 2;
-  static constexpr int kShort = sizeof(T) > 2 ? 4 : 2, kLong = 2, kUnroll = 1, kUnroll16 = 1, kCopy32 = 3, kCopy16 = 3;
+  static constexpr int kShort = sizeof(T) > 2 ? 4 : 2, kLong = 2, kUnroll = 1, kUnroll16 = sizeof(T) > 1 ? 2 : 1, kCopy32 = 3, kCopy16 = 3;
 };
 // FourCtas: the registers of TwoCtas in smaller CTAs (192 threads, four an SM).
 template <typename T> struct FourCtas : TwoCtas<T> {
