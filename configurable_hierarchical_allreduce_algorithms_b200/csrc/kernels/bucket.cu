@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "../api/chb.h"
+#include "common.cuh"
 
 namespace chb {
 
@@ -96,6 +97,7 @@ bucket_fill_kernel(BucketTable t, float* __restrict__ bucket) {
     else hi = mid - 1;
   }
   const int k = lo;
+  dependent_launch();
   const long long e0 = (long long)((int)blockIdx.x - t.first[k]) * kBucketBlock;
   float* dst = bucket + t.dst_off[k];
   const bool overwrite = (t.mode[k] & 1u) != 0;
@@ -135,8 +137,7 @@ int chb_bucket_fill(float* bucket, int count, const void* const* src, const long
     }
     t.first[t.count] = (int)ctas;
     if (ctas == 0) continue;
-    bucket_fill_kernel<<<(unsigned)ctas, kBucketThreads, 0, stream>>>(t, bucket);
-    if (cudaGetLastError() != cudaSuccess) return CHB_ERR_CUDA;
+    if (launch_overlapped(bucket_fill_kernel, dim3((unsigned)ctas), dim3(kBucketThreads), stream, t, bucket) != cudaSuccess) return CHB_ERR_CUDA;
   }
   return CHB_SUCCESS;
 }

@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(kLocalThreads)
 ag_local_kernel(World w, BulkIo io, long long nbytes) {
   constexpr int V = WIDE ? 32 : 16;
   const int P = w.P, owner = (int)blockIdx.y;
+  dependent_launch();
   const unsigned aborted = (int)threadIdx.x < P ? ld_volatile_u32(&w.ctrl[threadIdx.x]->abort) : 0u;   // (travels with the data)
   const long long nv = nbytes / V, j0 = (long long)blockIdx.x * (kLocalThreads * kLocalUnroll) + threadIdx.x;
   const char* src = io.in[owner];
@@ -261,9 +262,8 @@ int chb_ag_bulk(chb_comm* c, const void* const* in, void* const* out, long long 
     const bool wide = (low & 31ull) == 0ull;
     const long long piece = (long long)kLocalThreads * kLocalUnroll * (wide ? 32 : 16);
     const dim3 grid((unsigned)((nbytes + piece - 1) / piece), (unsigned)c->P, 1);
-    if (wide) ag_local_kernel<true><<<grid, kLocalThreads, 0, stream>>>(c->world, io, nbytes);
-    else ag_local_kernel<false><<<grid, kLocalThreads, 0, stream>>>(c->world, io, nbytes);
-    if (cudaGetLastError() != cudaSuccess) { c->last_error = "bulk allgather launch failed"; return CHB_ERR_CUDA; }
+    const cudaError_t e = launch_overlapped(wide ? ag_local_kernel<true> : ag_local_kernel<false>, grid, dim3(kLocalThreads), stream, c->world, io, nbytes);
+    if (e != cudaSuccess) { c->last_error = "bulk allgather launch failed"; return CHB_ERR_CUDA; }
     return CHB_SUCCESS;
   }
   const int max_pair_ctas = (kSigSlots - kSigNvlsBase) / kMaxRanks;

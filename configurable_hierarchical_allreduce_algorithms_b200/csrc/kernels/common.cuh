@@ -206,6 +206,28 @@ __device__ __forceinline__ bool cta_barrier(const World& w, Ctrl* c, int rank, u
   return s_ok != 0;
 }
 
+// ------------------------------------------------------------------ overlapped launches
+// A kernel that is usually launched right behind another one starts with dependent_launch(): its CTAs may be placed while
+// the grid before it in the stream drains (launch_overlapped), and wait here until that grid has completed and its writes
+// are visible.  Nothing of global memory may be touched before.
+__device__ __forceinline__ void dependent_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ------------------------------------------------------------------ element types
 
 template <typename T> struct Elem;  // acc type, elements per 16 bytes, conversions

@@ -116,6 +116,7 @@ constexpr int kLocalAdamThreads = 256;
 __global__ void __launch_bounds__(kLocalAdamThreads, 4)
 rs_adam_local_kernel(World w, AdamIo io, long long n, AdamHyper h) {
   const int P = w.P, rank = (int)blockIdx.y;
+  dependent_launch();
   const unsigned aborted = (int)threadIdx.x < P ? ld_volatile_u32(&w.ctrl[threadIdx.x]->abort) : 0u;   // (travels with the data)
   const long long nvec = n / 4, i = (long long)blockIdx.x * kLocalAdamThreads + threadIdx.x;
   const bool live = i < nvec;
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(kLocalAdamThreads)
 adam_flat_kernel(const float* __restrict__ grad, float* master, float* m, float* v, __nv_bfloat16* param,
                  long long n, AdamHyper h) {
   const long long i = (long long)blockIdx.x * kLocalAdamThreads + threadIdx.x;
+  dependent_launch();
   if (i >= n / 4) return;
   const float4 g = reinterpret_cast<const float4*>(grad)[i];
   float4 ww = reinterpret_cast<float4*>(master)[i], m1 = reinterpret_cast<float4*>(m)[i], v1 = reinterpret_cast<float4*>(v)[i];
@@ -228,8 +230,7 @@ int chb_rs_adam(chb_comm* c, const void* const* grad, void* const* master, void*
   AdamHyper h{hyper[0], hyper[1], hyper[2], hyper[3], hyper[4], hyper[5], hyper[6], hyper[7]};
   if (c->nlocal == c->P && !c->trace && !mc) {
     const dim3 grid((unsigned)((n / 4 + kLocalAdamThreads - 1) / kLocalAdamThreads), (unsigned)c->P, 1);
-    rs_adam_local_kernel<<<grid, kLocalAdamThreads, 0, stream>>>(c->world, io, n, h);
-    if (cudaGetLastError() != cudaSuccess) { c->last_error = "rs_adam launch failed"; return CHB_ERR_CUDA; }
+    if (launch_overlapped(rs_adam_local_kernel, grid, dim3(kLocalAdamThreads), stream, c->world, io, n, h) != cudaSuccess) { c->last_error = "rs_adam launch failed"; return CHB_ERR_CUDA; }
     return CHB_SUCCESS;
   }
   const int max_pair_ctas = (kSigSlots - kSigNvlsBase) / kMaxRanks;
@@ -256,9 +257,9 @@ int chb_adam_flat(const void* grad, void* master, void* m, void* v, void* param_
   if (n == 0) return CHB_SUCCESS;
   AdamHyper h{hyper[0], hyper[1], hyper[2], hyper[3], hyper[4], hyper[5], hyper[6], hyper[7]};
   const long long blocks = (n / 4 + kLocalAdamThreads - 1) / kLocalAdamThreads;
-  adam_flat_kernel<<<(unsigned)blocks, kLocalAdamThreads, 0, stream>>>((const float*)grad, (float*)master, (float*)m, (float*)v,
-                                                                   (__nv_bfloat16*)param_bf16, n, h);
-  return cudaGetLastError() == cudaSuccess ? CHB_SUCCESS : CHB_ERR_CUDA;
+  const cudaError_t e = launch_overlapped(adam_flat_kernel, dim3((unsigned)blocks), dim3(kLocalAdamThreads), stream, (const float*)grad,
+                                          (float*)master, (float*)m, (float*)v, (__nv_bfloat16*)param_bf16, n, h);
+  return e == cudaSuccess ? CHB_SUCCESS : CHB_ERR_CUDA;
 }
 
 }  // extern "C"

@@ -452,6 +452,7 @@ constexpr int kCopyCtasPerSm = 16;   // two waves of eight resident CTAs: measur
 // nvec: number of 32-byte vectors; src / dst 32-byte aligned.
 __global__ void __launch_bounds__(kCopyThreads)
 local_copy_kernel(Ctrl* c, const char* __restrict__ src, char* __restrict__ dst, long long nvec, int nrounds) {
+  dependent_launch();
   const long long tile = (long long)kCopyThreads * kCopyUnroll;
   const long long ntiles = (nvec + tile - 1) / tile;
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -569,8 +570,7 @@ int chb_run_program(chb_comm* c, const chb_program* p, int dtype, int op, const 
         const long long tiles = (nvec + kCopyThreads * kCopyUnroll - 1) / (kCopyThreads * kCopyUnroll);
         long long blocks = (long long)c->sm_count * kCopyCtasPerSm;
         if (blocks > tiles) blocks = tiles;
-        local_copy_kernel<<<(unsigned)blocks, kCopyThreads, 0, stream>>>(c->ctrl, sp, dp, nvec, g.nrounds);
-        if (cudaGetLastError() != cudaSuccess) { c->last_error = "copy launch failed"; return CHB_ERR_CUDA; }
+        if (launch_overlapped(local_copy_kernel, dim3((unsigned)blocks), dim3(kCopyThreads), stream, c->ctrl, sp, dp, nvec, g.nrounds) != cudaSuccess) { c->last_error = "copy launch failed"; return CHB_ERR_CUDA; }
         return CHB_SUCCESS;
       }
     }
