@@ -325,6 +325,7 @@ fp8_rs_local_kernel(World w, Fp8Io io, long long n, float out_scale) {
   __shared__ int s_ok;
   const int P = w.P;
   if (threadIdx.x == 0) s_ok = 1;
+  dependent_launch();
   __syncthreads();
   if ((int)threadIdx.x < P && ld_volatile_u32(&w.ctrl[threadIdx.x]->abort)) s_ok = 0;
   __syncthreads();
@@ -431,9 +432,8 @@ int chb_rs_fp8_wire(chb_comm* c, int dtype, const void* const* in, void* const* 
     long long ctas = (warps * 32 + kFuseThreads - 1) / kFuseThreads;
     const long long most = nctas > 0 ? (long long)nctas * c->P : (long long)c->sm_count * 4;      // resident at once
     if (ctas > most) ctas = most;
-    if (dtype == DT_F32) fp8_rs_local_kernel<float><<<(unsigned)ctas, kFuseThreads, 0, stream>>>(c->world, io, n, out_scale);
-    else fp8_rs_local_kernel<__nv_bfloat16><<<(unsigned)ctas, kFuseThreads, 0, stream>>>(c->world, io, n, out_scale);
-    if (cudaGetLastError() != cudaSuccess) { c->last_error = "fp8 reduce-scatter launch failed"; return CHB_ERR_CUDA; }
+    if (launch_overlapped(dtype == DT_F32 ? fp8_rs_local_kernel<float> : fp8_rs_local_kernel<__nv_bfloat16>, dim3((unsigned)ctas),
+                          dim3(kFuseThreads), stream, c->world, io, n, out_scale) != cudaSuccess) { c->last_error = "fp8 reduce-scatter launch failed"; return CHB_ERR_CUDA; }
     return CHB_SUCCESS;
   }
   const int max_pair_ctas = (kSigSlots - kSigNvlsBase) / kMaxRanks;

@@ -96,6 +96,7 @@ lock_tiny_kernel(World w, const char* __restrict__ blob, int blob_bytes, IoTable
   __shared__ int s_ok;
   const int tid = threadIdx.x;
   if (tid == 0) s_ok = 1;
+  dependent_launch();
   __syncthreads();
   if (tid < w.P && ld_volatile_u32(&w.ctrl[tid]->abort)) s_ok = 0;
   {
@@ -168,6 +169,7 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
   const int tid = threadIdx.x;
   const long long nct = gridDim.x, cta = blockIdx.x;
   if (tid == 0) s_ok = 1;
+  dependent_launch();
   __syncthreads();
   if (tid < w.P && ld_volatile_u32(&w.ctrl[tid]->abort)) s_ok = 0;
   const char* tab = blob;
@@ -416,33 +418,38 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
   unsigned long long low = (unsigned long long)b.grid * esz;             // low bits of every address and length
   for (int l = 0; l < c->P; ++l) low |= (unsigned long long)(uintptr_t)in[l] | (unsigned long long)(uintptr_t)out[l];
   const bool vec = (low & 15ull) == 0ull;
+  void* tiny_args[] = {&w, &bp, &bytes, &io, &op, &scale};
+  void* wide_args[] = {&w, &bp, &bytes, &in_smem, &io, &op, &scale};
+  const size_t smem = in_smem ? (size_t)b.bytes : 0;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2] = {};
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.dynamicSmemBytes = smem;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see dependent_launch()
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 1;
   if (nctas <= 0 && b.accesses <= kTinyAccesses * b.nrounds * (vec ? 16 / (long long)esz : 1) && tiny_smem <= (size_t)kLockSmemTables) {
-    void* args[] = {&w, &bp, &bytes, &io, &op, &scale};
-    e = cudaLaunchKernel(vec ? fn.tiny_vec : fn.tiny, dim3(1), dim3(kTinyThreads), args, tiny_smem, stream);
+    cfg.gridDim = dim3(1);
+    cfg.blockDim = dim3(kTinyThreads);
+    cfg.dynamicSmemBytes = tiny_smem;
+    e = cudaLaunchKernelExC(&cfg, vec ? fn.tiny_vec : fn.tiny, tiny_args);
+  } else if (b.nrounds > 1 && n > 1 && (n <= kLockCluster || (nctas <= 0 && b.max_grains <= kClusterGrains))) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)(n < kLockCluster ? n : kLockCluster);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+    cfg.gridDim = dim3(attr[1].val.clusterDim.x);
+    cfg.blockDim = dim3(OneCta<float>::kThreads);
+    e = cudaLaunchKernelExC(&cfg, fn.cluster, wide_args);
   } else {
-    void* args[] = {&w, &bp, &bytes, &in_smem, &io, &op, &scale};
-    const size_t smem = in_smem ? (size_t)b.bytes : 0;
-    const void* wide = two ? fn.wide2 : fn.wide;
-    const dim3 block(two ? TwoCtas<float>::kThreads : OneCta<float>::kThreads);
-    const bool cluster = b.nrounds > 1 && n > 1 && (n <= kLockCluster || (nctas <= 0 && b.max_grains <= kClusterGrains));
-    if (cluster) {
-      cudaLaunchConfig_t cfg{};
-      cudaLaunchAttribute attr{};
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = (unsigned)(n < kLockCluster ? n : kLockCluster);
-      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-      cfg.gridDim = dim3(attr.val.clusterDim.x);
-      cfg.blockDim = dim3(OneCta<float>::kThreads);
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = stream;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      e = cudaLaunchKernelExC(&cfg, fn.cluster, args);
-    } else if (b.nrounds > 1 && n > 1) {
-      e = cudaLaunchCooperativeKernel(wide, dim3((unsigned)n), block, args, smem, stream);
-    } else {
-      e = cudaLaunchKernel(wide, dim3((unsigned)n), block, args, smem, stream);
+    cfg.gridDim = dim3((unsigned)n);
+    cfg.blockDim = dim3(two ? TwoCtas<float>::kThreads : OneCta<float>::kThreads);
+    if (b.nrounds > 1 && n > 1) {      // CTAs that wait for each other
+      attr[0].id = cudaLaunchAttributeCooperative;
+      attr[0].val.cooperative = 1;
     }
+    e = cudaLaunchKernelExC(&cfg, two ? fn.wide2 : fn.wide, wide_args);
   }
   if (e != cudaSuccess) {
     c->last_error = std::string("lockstep launch failed: ") + cudaGetErrorString(e);
