@@ -79,7 +79,7 @@ int chb_program_ll_info(const chb_program_t* p, int esz, long long* info, int n)
 int chb_program_simulate_ll(const chb_program_t* p, int dtype, int op, void* const* in, void* const* out,
                             uint64_t seed, int nthreads, int fault, int launches, char* err, int errlen);
 /* The lockstep form (one grid runs all ranks, see sched/lock_plan.h); rewrite: 0 the steps as lowered, 1 copies rewritten
- * (16-bit floats), 2 also chains of reductions joined (all other types).
+ * (16-bit floats and bytes), 2 also chains of reductions joined (all other types).
  * chb_program_lock_info: info = rounds, steps, elements read, elements stored.
  * chb_program_simulate_lock: run it on host buffers, the steps of a round in a random order (seed); two steps of one
  *   round that touch the same memory end the run with CHB_ERR_TIMEOUT and their round in err. */

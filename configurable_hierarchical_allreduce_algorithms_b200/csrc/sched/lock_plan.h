@@ -43,9 +43,9 @@ struct LockPlan {
 
 // rewrite: LOCK_PLAIN only the layout (for comparing), LOCK_COPIES without rewrite 3, LOCK_CHAINS everything.
 enum { LOCK_PLAIN = 0, LOCK_COPIES = 1, LOCK_CHAINS = 2 };
-// The rewriting for a stored type: 16-bit floats are rounded after every step, the others accumulate in themselves
-// (bytes in 32 bits, which agrees modulo 256).
-inline int lock_rewrite_for(int dtype) { return dtype == DT_BF16 || dtype == DT_F16 ? LOCK_COPIES : LOCK_CHAINS; }
+// The rewriting for a stored type: the 16-bit floats are rounded and bytes wrap after every step (which a scale would
+// show), the others accumulate in themselves.
+inline int lock_rewrite_for(int dtype) { return dtype == DT_BF16 || dtype == DT_F16 || dtype == DT_U8 ? LOCK_COPIES : LOCK_CHAINS; }
 LockPlan make_lock_plan(const Program& p, int rewrite);
 
 // Device tables: LockHeader, LockRound[nrounds], LockStep[nsteps], LockRef[nrefs] (a step's sources, then its

@@ -46,6 +46,19 @@ def test_lockstep_equals_pull(cuda, coll, P, k, b):
     comm.close()
 
 
+def test_bytes_wrap_after_every_step(cuda):
+    """A chain of byte additions is not joined: its partial sums wrap, which a scale brings to light."""
+    P, n = 4, 5000
+    comm = Communicator.emulated(P, scratch_bytes=4 << 20, user_bytes=4096)
+    src = [torch.randint(0, 256, (P * n,), device="cuda", dtype=torch.int32).to(torch.uint8) for _ in range(P)]
+    for name in ("ring", "pairwise"):
+        want = chb.reduce_scatter(comm, src, algo=name + ":pull", scale=0.5)
+        got = chb.reduce_scatter(comm, src, algo=name, scale=0.5)
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), name
+    comm.check()
+    comm.close()
+
+
 def test_lockstep_in_place_and_overlapping_buffers(cuda):
     P, n = 4, 5003
     comm = Communicator.emulated(P, scratch_bytes=4 << 20, user_bytes=4096)
