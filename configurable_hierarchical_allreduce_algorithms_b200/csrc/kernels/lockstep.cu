@@ -157,6 +157,35 @@ lock_tiny_kernel(World w, const char* __restrict__ blob, int blob_bytes, IoTable
   }
 }
 
+// A span whose destinations lie on different 16-byte grids and several of which are its sources (an in-place allreduce of
+// skewed buffers): every thread reads all sources of its elements, kElementUnroll at a time, before it stores any.
+// Bound by the requests of element-wise accesses.  8 ranks in place, fp32 25 MB, k = 4, b = 2: 109 us where all buffers are
+// aligned, 223 us here (994 us with the per-rank kernels).
+constexpr int kElementUnroll = 4;
+template <typename T>
+__device__ __forceinline__ void element_span(const SpanArgs* a) {
+  using Acc = typename Elem<T>::Acc;
+  const long long count = a->count, nt = blockDim.x;
+  for (long long e0 = threadIdx.x; e0 < count; e0 += nt * kElementUnroll) {
+    Acc v[kElementUnroll];
+#pragma unroll
+    for (int u = 0; u < kElementUnroll; ++u) v[u] = e0 + u * nt < count ? Elem<T>::up(__ldcg(reinterpret_cast<const T*>(a->src[0]) + e0 + u * nt)) : (Acc)0;
+#pragma unroll 2
+    for (int s = 1; s < a->nsrc; ++s) {
+      const T* src = reinterpret_cast<const T*>(a->src[s]) + e0;
+#pragma unroll
+      for (int u = 0; u < kElementUnroll; ++u)
+        if (e0 + u * nt < count) v[u] = combine<Acc>(a->op, v[u], Elem<T>::up(__ldcg(src + u * nt)));
+    }
+#pragma unroll
+    for (int u = 0; u < kElementUnroll; ++u) {
+      if (a->do_scale) v[u] = (Acc)(v[u] * a->scale);
+      if (e0 + u * nt < count)
+        for (int d = 0; d < a->ndst; ++d) reinterpret_cast<T*>(a->dst[d])[e0 + u * nt] = Elem<T>::down(v[u]);
+    }
+  }
+}
+
 // CLUSTER: the grid is one cluster (small messages), else the CTAs are co-resident by a cooperative launch, or the schedule
 // has one round only.
 template <typename T, bool CLUSTER, typename Shape>
@@ -208,19 +237,18 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
         const unsigned grid16 = (unsigned)(reinterpret_cast<unsigned long long>(p) & 15ull);
         const unsigned first16 = __shfl_sync(0xffffffffu, grid16, kept ? __ffs((int)kept) - 1 : 0);
         const bool mixed = __any_sync(0xffffffffu, keep && grid16 != first16);
-        // one destination at a time re-reads the sources, so the one that is a source itself comes last
         bool is_src = false;
         if (mixed && keep)
           for (int j = 0; j < st.nsrc; ++j) {
             const LockRef x = refs[st.ref_begin + j];
             is_src = is_src || p == lock_base(w, io, x.rank, x.buf) + (x.off + e0) * (long long)sizeof(T);
           }
-        const unsigned last = __ballot_sync(0xffffffffu, is_src);
+        const unsigned sources = __ballot_sync(0xffffffffu, is_src);
         const int n = __popc(kept);
-        const int at = is_src ? n - 1 : __popc(kept & ~last & ((1u << tid) - 1u));
+        const int at = lock_slot(tid, kept, mixed, sources);
         if (keep) { s_dst[at] = p; s_span.dst[at] = p; }
         if (tid == 0) {
-          s_passes = mixed ? n : (n ? 1 : 0);
+          s_passes = lock_passes(kept, mixed, sources);
           s_span.nsrc = st.nsrc;
           s_span.ndst = n;
           s_span.count = e1 - e0;
@@ -250,7 +278,8 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
   __syncthreads();
   for (int t = 0; t < nrounds; ++t) {
     while (i >= 0) {
-      const int passes = s_passes;           // more than one: destinations on different 16-byte grids, one at a time
+      const int passes = s_passes;           // see lock_passes()
+      if (passes < 0) element_span<T>(&s_span);
       for (int d = 0; d < passes; ++d) {
         if (passes > 1) {
           __syncthreads();

@@ -336,12 +336,41 @@ int simulate_lock_t(const Program& p, const LockPlan& plan, int rop, void* const
         }
     std::shuffle(now.begin(), now.end(), rng);
     for (const LockStepPlan& x : now) {
-      std::vector<T> v(ptr(x.srcs[0].peer, x.srcs[0].buf, x.srcs[0].off), ptr(x.srcs[0].peer, x.srcs[0].buf, x.srcs[0].off) + x.count);
-      for (size_t i = 1; i < x.srcs.size(); ++i) {
-        const T* y = ptr(x.srcs[i].peer, x.srcs[i].buf, x.srcs[i].off);
-        for (int64_t e = 0; e < x.count; ++e) v[(size_t)e] = combine_host<T>(rop, v[(size_t)e], y[e]);
+      auto combined = [&] {
+        const T* first = ptr(x.srcs[0].peer, x.srcs[0].buf, x.srcs[0].off);
+        std::vector<T> v(first, first + x.count);
+        for (size_t i = 1; i < x.srcs.size(); ++i) {
+          const T* y = ptr(x.srcs[i].peer, x.srcs[i].buf, x.srcs[i].off);
+          for (int64_t e = 0; e < x.count; ++e) v[(size_t)e] = combine_host<T>(rop, v[(size_t)e], y[e]);
+        }
+        return v;
+      };
+      unsigned kept = 0u, sources = 0u;
+      bool mixed = false;
+      T* to[kLockMaxDst] = {};
+      T* slot[kLockMaxDst] = {};
+      uintptr_t grid = 0;
+      for (size_t q = 0; q < x.dsts.size(); ++q) {
+        to[q] = ptr(x.dsts[q].rank, x.dsts[q].buf, x.dsts[q].off);
+        if (x.srcs.size() == 1 && !x.final && to[q] == ptr(x.srcs[0].peer, x.srcs[0].buf, x.srcs[0].off)) continue;
+        if (kept == 0u) grid = (uintptr_t)to[q] & 15u;
+        mixed = mixed || ((uintptr_t)to[q] & 15u) != grid;
+        kept |= 1u << q;
+        for (const Src& r : x.srcs)
+          if (ptr(r.peer, r.buf, r.off) == to[q]) sources |= 1u << q;
       }
-      for (const LockDst& d : x.dsts) std::memcpy(ptr(d.rank, d.buf, d.off), v.data(), (size_t)x.count * sizeof(T));
+      for (size_t q = 0; q < x.dsts.size(); ++q)
+        if ((kept >> q) & 1u) slot[lock_slot((int)q, kept, mixed, sources)] = to[q];
+      const int passes = lock_passes(kept, mixed, sources);
+      std::vector<T> v;
+      for (int d = 0; d < lock_bits(kept); ++d) {
+        if (!slot[d]) {
+          if (err) *err = "a step of round " + std::to_string(x.level) + " of " + p.name + " leaves a destination unset";
+          return -1;
+        }
+        if (d == 0 || passes > 1) v = combined();
+        std::memcpy(slot[d], v.data(), (size_t)x.count * sizeof(T));
+      }
     }
     a = b;
   }

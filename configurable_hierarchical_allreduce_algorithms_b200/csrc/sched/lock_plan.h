@@ -48,6 +48,36 @@ enum { LOCK_PLAIN = 0, LOCK_COPIES = 1, LOCK_CHAINS = 2 };
 inline int lock_rewrite_for(int dtype) { return dtype == DT_BF16 || dtype == DT_F16 || dtype == DT_U8 ? LOCK_COPIES : LOCK_CHAINS; }
 LockPlan make_lock_plan(const Program& p, int rewrite);
 
+// How a CTA stores the destinations of a step that it has to write (one bit each in `kept`; a copy onto itself is not
+// kept).  mixed: they lie on different 16-byte grids, which the vector loops cannot serve at once; `sources`: those that
+// are a source of the step as well (same address), looked at only where mixed.
+//   0  nothing to store          1  one span for all
+//   n  a span for each of the n, which reads the sources anew, so that the one that is a source has to be the last
+//  -1  element by element, every source read before any destination is written: several are sources (an in-place
+//      allreduce whose chains were joined), and each pass but the first would read what the one before it has stored
+#ifdef __CUDACC__
+#define CHB_HOST_DEVICE __host__ __device__
+#else
+#define CHB_HOST_DEVICE
+#endif
+CHB_HOST_DEVICE inline int lock_bits(unsigned m) {
+#ifdef __CUDA_ARCH__
+  return __popc(m);
+#else
+  return __builtin_popcount(m);
+#endif
+}
+CHB_HOST_DEVICE inline int lock_passes(unsigned kept, bool mixed, unsigned sources) {
+  if (kept == 0u) return 0;
+  if (!mixed) return 1;
+  return lock_bits(kept & sources) > 1 ? -1 : lock_bits(kept);
+}
+// Place of destination i among the kept ones.
+CHB_HOST_DEVICE inline int lock_slot(int i, unsigned kept, bool mixed, unsigned sources) {
+  const unsigned last = lock_passes(kept, mixed, sources) > 1 ? kept & sources : 0u;
+  return (last >> i) & 1u ? lock_bits(kept) - 1 : lock_bits(kept & ~last & ((1u << i) - 1u));
+}
+
 // Device tables: LockHeader, LockRound[nrounds], LockStep[nsteps], LockRef[nrefs] (a step's sources, then its
 // destinations).  prefix: cost of the round's earlier steps; the cost of a step is its grains x (sources + destinations).
 // elems: elements of the round's earlier steps.
@@ -58,8 +88,8 @@ struct LockRef { long long off; int rank, buf; };
 static_assert(sizeof(LockHeader) % 16 == 0 && sizeof(LockRound) % 16 == 0 && sizeof(LockStep) % 16 == 0 && sizeof(LockRef) % 16 == 0, "copied as 16-byte words");
 std::vector<char> make_lock_blob(const LockPlan& p);
 
-// Executes the plan on host memory, the steps of a round in random order, and checks that no step of a round touches
-// what another one writes.  Returns 0, -1 (err says what) or -2 for a bad argument.
+// Executes the plan on host memory, the steps of a round in random order and the destinations of a step as lock_passes
+// has them stored at these addresses, and checks that no step of a round touches what another one writes.  Returns 0, -1 (err says what) or -2 for a bad argument.
 int simulate_lock(const Program& p, int dtype, int op, void* const* in, void* const* out, uint64_t seed,
                   int rewrite, std::string* err);
 

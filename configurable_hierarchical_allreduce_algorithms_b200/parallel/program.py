@@ -170,21 +170,28 @@ class Program:
         return [o[:self.out_elems] for o in outs]
 
     def simulate_lock(self, inputs: list[np.ndarray], op: str = "sum", seed: int = 0, rewrite: int = 2,
-                      alias: bool = False) -> list[np.ndarray]:
+                      alias: bool = False, skew=None) -> list[np.ndarray]:
         """Run the lockstep form (all ranks executed by one grid, ``csrc/sched/lock_plan.h``) on host arrays, the steps
         of a round in random order.  ``rewrite``: 0 leaves the program's steps as lowered, 1 rewrites copies, 2 also joins
-        chains of reductions; ``alias`` as in :meth:`simulate`."""
+        chains of reductions; ``alias`` as in :meth:`simulate`; ``skew``: elements by which each rank's buffers start
+        beyond a 16-byte boundary."""
         assert len(inputs) == self.P
         dt = np.dtype(inputs[0].dtype)
         poison = 239 if dt.kind == "u" else -17
+        skew = skew or [0] * self.P
+
+        def buffer(n, r):
+            raw = np.full(n + skew[r] + 16, poison, dtype=dt)
+            at = -raw.ctypes.data % 16 // dt.itemsize + skew[r]
+            return raw[at:at + n]
+
         if alias:
             assert self.in_place, "aliased buffers need a program lowered with in_place=True"
-            ins = outs = [np.full(max(self.in_elems, self.out_elems), poison, dtype=dt) for _ in range(self.P)]
-            for buf, x in zip(ins, inputs):
-                buf[:x.size] = x
+            ins = outs = [buffer(max(self.in_elems, self.out_elems), r) for r in range(self.P)]
         else:
-            ins = [np.ascontiguousarray(x, dtype=dt) for x in inputs]
-            outs = [np.full(self.out_elems, poison, dtype=dt) for _ in range(self.P)]
+            ins, outs = [buffer(x.size, r) for r, x in enumerate(inputs)], [buffer(self.out_elems, r) for r in range(self.P)]
+        for buf, x in zip(ins, inputs):
+            buf[:x.size] = x
         ip = (C.c_void_p * self.P)(*[x.ctypes.data for x in ins])
         opp = (C.c_void_p * self.P)(*[x.ctypes.data for x in outs])
         err = C.create_string_buffer(512)

@@ -165,3 +165,37 @@ def test_automatic_small_calls_equal_the_line_kernels(cuda, P):
         torch.testing.assert_close(y, full, rtol=1e-5, atol=1e-5 * P)
     comm.check()
     comm.close()
+
+
+@pytest.mark.parametrize("P,algo,k,b", [(3, "ring", 2, 1), (4, "ring", 2, 1), (8, "ring", 2, 1), (4, "radix_batch", 2, 2), (8, "radix_batch", 4, 2),
+                                        (8, "radix_batch", 2, 2), (8, "radix_batch", 4, 4), (8, "radix_batch", 2, 1)])
+def test_in_place_on_different_16_byte_grids(cuda, P, algo, k, b):
+    """Steps that store to several of their own operands, which skewed buffers keep from one vector loop: one CTA, a
+    cluster and the whole grid, against the pull interpreter, and nothing written around the buffers."""
+    comm = Communicator.emulated(P, scratch_bytes=24 << 20, user_bytes=4096)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    for n in (24 * P, 2049 * P, 150_001 * P):
+        for dtype in (torch.float32, torch.int32) if n > 24 * P else (torch.float32, torch.float64, torch.bfloat16):
+            for skew in ([r % 4 for r in range(P)], [0] * (P - 1) + [1]):
+                src = [torch.rand(n, generator=g, device="cuda").mul_(99).to(dtype) for _ in range(P)]
+                want = chb.all_reduce(comm, src, algo=algo + ":pull", k=k, b=b)
+                full = [torch.zeros(n + 4, dtype=dtype, device="cuda") for _ in range(P)]
+                bufs = [f[a:a + n] for f, a in zip(full, skew)]
+                for x, s in zip(bufs, src):
+                    x.copy_(s)
+                chb.all_reduce(comm, bufs, out=bufs, algo=algo, k=k, b=b)
+                for r in range(P):
+                    assert torch.equal(bufs[r], want[r]), (n, dtype, skew, r)
+                    assert not full[r][:skew[r]].any() and not full[r][skew[r] + n:].any()
+    comm.check()
+    comm.close()
+
+
+def test_automatic_in_place_on_the_rows_of_an_odd_matrix(cuda):
+    comm = Communicator.emulated(8, scratch_bytes=80 << 20, user_bytes=4096)
+    m = torch.randn(8, 2_000_001, device="cuda")
+    want = chb.all_reduce(comm, list(m.clone()), algo="ring:pull")
+    chb.all_reduce(comm, list(m), out=list(m))
+    assert all(torch.equal(x, y) for x, y in zip(m, want))
+    comm.check()
+    comm.close()

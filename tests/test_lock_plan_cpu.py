@@ -54,3 +54,25 @@ def test_rewriting_removes_the_passes_it_is_for():
     for algo in ("pairwise", "ring"):
         i = chb.Program("reduce_scatter", algo, P, 100, 2, 1).lock_info()
         assert (i["rounds"], i["reads"], i["stores"]) == (1, P * P * 100, P * 100), (algo, i)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.int32, np.float64])
+@pytest.mark.parametrize("algo", ["ring", "radix_batch", "recursive_doubling", "reduce_scatter_allgather"])
+def test_in_place_on_different_16_byte_grids(algo, dtype):
+    """Joined chains of an in-place allreduce store to several of their own operands; with the ranks' buffers on different
+    16-byte grids no single vector loop serves those, and none may be read after it has been overwritten."""
+    rng = np.random.default_rng(5)
+    several = 0
+    for P, k, b in ((3, 2, 1), (4, 2, 2), (4, 4, 1), (8, 4, 2), (8, 2, 2), (8, 4, 4), (8, 2, 1), (12, 3, 4), (16, 4, 4)):
+        for low in (dict(in_place=True), dict(in_place=True, in_symmetric=True, out_symmetric=True)):
+            p = chb.Program("allreduce", algo, P, 37 * P, k, b, **low)
+            ins = [rng.standard_normal(p.in_elems) * 9 for _ in range(P)]
+            ins = [x.astype(dtype) for x in ins]
+            want = p.simulate([x.copy() for x in ins], alias=True)
+            for skew in ([r % 4 for r in range(P)], [0] * (P - 1) + [1], [(3 * r + 1) % 4 for r in range(P)]):
+                for rewrite in (0, 1, 2):
+                    got = p.simulate_lock(ins, seed=k, rewrite=rewrite, alias=True, skew=skew)
+                    for r in range(P):
+                        assert got[r].tobytes() == want[r].tobytes(), (P, k, b, low, skew, rewrite, r)
+                several += 1
+    assert several
