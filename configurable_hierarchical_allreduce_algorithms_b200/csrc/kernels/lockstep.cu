@@ -157,8 +157,8 @@ lock_tiny_kernel(World w, const char* __restrict__ blob, int blob_bytes, IoTable
   }
 }
 
-// A span whose destinations lie on different 16-byte grids and several of which are its sources (an in-place allreduce of
-// skewed buffers): every thread reads all sources of its elements, kElementUnroll at a time, before it stores any.
+// A span whose destinations lie on different 16-byte grids and that is short, or several of whose destinations are its sources
+// (an in-place allreduce of skewed buffers): every thread reads all sources of its elements, kElementUnroll at a time, before it stores any.
 // Bound by the requests of element-wise accesses.  8 ranks in place, fp32 25 MB, k = 4, b = 2: 109 us where all buffers are
 // aligned, 223 us here (994 us with the per-rank kernels).
 constexpr int kElementUnroll = 4;
@@ -245,10 +245,10 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
           }
         const unsigned sources = __ballot_sync(0xffffffffu, is_src);
         const int n = __popc(kept);
-        const int at = lock_slot(tid, kept, mixed, sources);
+        const int at = lock_slot(tid, kept, mixed, sources, e1 - e0);
         if (keep) { s_dst[at] = p; s_span.dst[at] = p; }
         if (tid == 0) {
-          s_passes = lock_passes(kept, mixed, sources);
+          s_passes = lock_passes(kept, mixed, sources, e1 - e0);
           s_span.nsrc = st.nsrc;
           s_span.ndst = n;
           s_span.count = e1 - e0;

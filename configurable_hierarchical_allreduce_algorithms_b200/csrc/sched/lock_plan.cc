@@ -360,8 +360,8 @@ int simulate_lock_t(const Program& p, const LockPlan& plan, int rop, void* const
           if (ptr(r.peer, r.buf, r.off) == to[q]) sources |= 1u << q;
       }
       for (size_t q = 0; q < x.dsts.size(); ++q)
-        if ((kept >> q) & 1u) slot[lock_slot((int)q, kept, mixed, sources)] = to[q];
-      const int passes = lock_passes(kept, mixed, sources);
+        if ((kept >> q) & 1u) slot[lock_slot((int)q, kept, mixed, sources, x.count)] = to[q];
+      const int passes = lock_passes(kept, mixed, sources, x.count);
       std::vector<T> v;
       for (int d = 0; d < lock_bits(kept); ++d) {
         if (!slot[d]) {

@@ -199,3 +199,24 @@ def test_automatic_in_place_on_the_rows_of_an_odd_matrix(cuda):
     assert all(torch.equal(x, y) for x, y in zip(m, want))
     comm.check()
     comm.close()
+
+
+@pytest.mark.parametrize("coll", ["allreduce", "allgather"])
+def test_skewed_destinations_around_the_longest_element_wise_span(cuda, coll):
+    """One CTA a rank, so that a step of the round is one span: element by element up to 8192 elements, a pass for each
+    destination beyond."""
+    P = 3
+    comm = Communicator.emulated(P, ll_bytes=64 << 10, scratch_bytes=4 << 20, user_bytes=4096)
+    for blk in (8191, 8192, 8193, 10241):
+        n_in, n_out = lengths(coll, P, blk)
+        for dtype in (torch.float32, torch.bfloat16):
+            ins = [torch.randn(n_in + 2, device="cuda").to(dtype)[r:r + n_in] for r in range(P)]
+            full = [torch.zeros(n_out + 4, dtype=dtype, device="cuda") for _ in range(P)]
+            outs = [f[r:r + n_out] for r, f in enumerate(full)]
+            want = FNS[coll](comm, ins, algo="radix_batch:pull")
+            FNS[coll](comm, ins, out=outs, algo="radix_batch", nctas=1)
+            for r in range(P):
+                assert torch.equal(outs[r], want[r]), (blk, dtype, r)
+                assert not full[r][:r].any() and not full[r][r + n_out:].any()
+    comm.check()
+    comm.close()
