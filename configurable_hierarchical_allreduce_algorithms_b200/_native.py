@@ -61,6 +61,8 @@ def _declare(L: C.CDLL) -> None:
     L.chb_program_lock_info.argtypes = [vp, i32, C.POINTER(C.c_longlong), i32]
     L.chb_program_simulate_lock.restype = i32
     L.chb_program_simulate_lock.argtypes = [vp, i32, i32, C.POINTER(vp), C.POINTER(vp), u64, i32, cp, i32]
+    L.chb_simulate_flat.restype = i32
+    L.chb_simulate_flat.argtypes = [i32, i32, i32, i32, C.POINTER(vp), C.POINTER(vp), C.c_longlong, u64, cp, i32]
     L.chb_program_export.restype = i32
     L.chb_program_export.argtypes = [vp, vp, vp, vp, vp, vp]
     L.chb_list_algorithms.restype = i32

@@ -86,6 +86,10 @@ int chb_program_simulate_ll(const chb_program_t* p, int dtype, int op, void* con
 int chb_program_lock_info(const chb_program_t* p, int rewrite, long long* info, int n);
 int chb_program_simulate_lock(const chb_program_t* p, int dtype, int op, void* const* in, void* const* out,
                               uint64_t seed, int rewrite, char* err, int errlen);
+/* The same for the flat schedule of an allreduce, reduce-scatter or allgather (count as in chb_collective), which has no
+ * program. */
+int chb_simulate_flat(int coll, int P, int dtype, int op, void* const* in, void* const* out, long long count, uint64_t seed,
+                      char* err, int errlen);
 /* run all ranks as host threads (real concurrency); mean wall seconds per repetition in *seconds */
 int chb_program_run_threads(const chb_program_t* p, int dtype, int op, void* const* in, void* const* out,
                             int iters, double* seconds);

@@ -25,6 +25,8 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
                              void* const* out, float scale, int nctas, cudaStream_t stream);
 int chb_lockstep_ok(const chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out,
                     long long slot_bytes);
+int chb_run_flat_lockstep(chb_comm* c, int coll, int dtype, int op, const void* const* in, void* const* out, long long n,
+                          float scale, cudaStream_t stream);
 int chb_program_fits(const chb_comm* c, const chb_program* p, int dtype);
 int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, long long payload_bytes);
 long long chb_program_ll_lines(const chb_program* p, int esz);
@@ -85,9 +87,6 @@ bool all_symmetric(const chb_comm* c, const void* const* ptrs) {
   return true;
 }
 
-constexpr int kFlatProgram = 8;     // a flag of get_program: the program of flat_builder instead of a named algorithm's
-chb::Builder flat_builder(int coll, int P, int64_t n);
-
 int get_program(chb_comm* c, int coll, const char* algo, int k, int b, int aux, int64_t count, int flags,
                 chb_program** out) {
   Key key(coll, algo, k, b, aux, count, flags);
@@ -109,7 +108,7 @@ int get_program(chb_comm* c, int coll, const char* algo, int k, int b, int aux, 
     s.b = b;
     s.count = count;
     s.aux = aux;
-    chb::Builder B = flags & kFlatProgram ? flat_builder(coll, c->P, count) : chb::build_algorithm(s);
+    chb::Builder B = chb::build_algorithm(s);
     chb::LowerOpts o;
     o.in_symmetric = (flags & 1) != 0;
     o.out_symmetric = (flags & 2) != 0;
@@ -123,24 +122,6 @@ int get_program(chb_comm* c, int coll, const char* algo, int k, int b, int aux, 
     c->last_error = e.what();
     return c->last_error.find("count") != std::string::npos ? CHB_ERR_COUNT : CHB_ERR_ARG;
   }
-}
-
-// What the one-shot and two-shot line kernels compute, as a program: operands in rank order, every rank the same result.
-// Used only in lockstep (all ranks on this GPU), where the rewriting makes one step of it, so nothing is sliced and any
-// length will do.
-chb::Builder flat_builder(int coll, int P, int64_t n) {
-  const int64_t ni = coll == CHB_REDUCE_SCATTER ? n * P : n, no = coll == CHB_ALLGATHER ? n * P : n;
-  chb::Builder B(P, ni, no, "flat");
-  std::vector<chb::Src> srcs((size_t)P);
-  for (int r = 0; r < P; ++r) {
-    for (int q = 0; q < P; ++q) srcs[(size_t)q] = chb::Src{q, chb::L_IN, coll == CHB_REDUCE_SCATTER ? r * n : 0};
-    if (coll == CHB_REDUCE_SCATTER) B.reduce(r, chb::L_OUT, 0, srcs, n, false, chb::OPF_FINAL);
-    else if (coll == CHB_ALLREDUCE && r == 0) B.reduce(0, chb::L_OUT, 0, srcs, n, false, chb::OPF_FINAL);
-    else if (coll == CHB_ALLREDUCE) B.copy(r, chb::L_OUT, 0, 0, chb::L_OUT, 0, n);
-    else
-      for (int q = 0; q < P; ++q) B.copy(r, chb::L_OUT, q * n, q, chb::L_IN, 0, n);
-  }
-  return B;
 }
 
 }  // namespace
@@ -271,11 +252,7 @@ int chb_collective_local(chb_comm* c, int coll, int two_shot, int dtype, int op,
   for (int r = 0; r < c->P; ++r) low |= (uintptr_t)in[r] | (uintptr_t)out[r];
   const long long nbytes = (long long)count * chb_dtype_size(dtype);
   if ((low & 7u) || nbytes > (two_shot ? chb_ll2_max_bytes(c) : chb_ll_max_bytes(c)) || (two_shot && coll != CHB_ALLREDUCE)) return CHB_ERR_UNSUPPORTED;
-  chb_program* p = nullptr;
-  const int rc = get_program(c, coll, "", 0, 0, 0, count, kFlatProgram | 3, &p);
-  if (rc) return rc;
-  if (!chb_lockstep_ok(c, p, dtype, in, out, coll == CHB_ALLGATHER ? nbytes : 0)) return CHB_ERR_UNSUPPORTED;
-  return chb_run_program_lockstep(c, p, dtype, op, in, out, scale, 0, stream);
+  return chb_run_flat_lockstep(c, coll, dtype, op, in, out, count, scale, stream);
 }
 
 // ---------------------------------------------------------------- reference-compatible calls

@@ -167,6 +167,15 @@ int chb_program_simulate_lock(const chb_program_t* p, int dtype, int op, void* c
   return CHB_SUCCESS;
 }
 
+int chb_simulate_flat(int coll, int P, int dtype, int op, void* const* in, void* const* out, long long count, uint64_t seed,
+                      char* err, int errlen) {
+  if (coll < 0 || coll > 2 || P < 1 || P > chb::kLockMaxDst || count <= 0 || !in || !out) return CHB_ERR_ARG;
+  std::string e;
+  const int rc = chb::simulate_flat(chb::FlatSpec{coll, 0, count}, P, dtype, op, in, out, seed, &e);
+  if (rc) { set_err(err, errlen, e); return rc == -1 ? CHB_ERR_TIMEOUT : CHB_ERR_ARG; }
+  return CHB_SUCCESS;
+}
+
 int chb_program_run_threads(const chb_program_t* p, int dtype, int op, void* const* in, void* const* out,
                             int iters, double* seconds) {
   if (!p || !in || !out) return CHB_ERR_ARG;

@@ -89,7 +89,7 @@ __device__ __forceinline__ char* lock_base(const World& w, const IoTable& io, in
 // the launch need not be cooperative.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kTinyThreads, 1)
-lock_tiny_kernel(World w, const char* __restrict__ blob, int blob_bytes, IoTable io, int op, float scale) {
+lock_tiny_kernel(World w, const char* __restrict__ blob, int blob_bytes, FlatSpec flat, IoTable io, int op, float scale) {
   using Acc = typename Elem<T>::Acc;
   constexpr int VE = VEC ? Elem<T>::kPerVec : 1;
   extern __shared__ __align__(16) unsigned char lock_tables[];
@@ -99,7 +99,9 @@ lock_tiny_kernel(World w, const char* __restrict__ blob, int blob_bytes, IoTable
   dependent_launch();
   __syncthreads();
   if (tid < w.P && ld_volatile_u32(&w.ctrl[tid]->abort)) s_ok = 0;
-  {
+  if (flat.coll >= 0) {
+    flat_write(flat, w.P, reinterpret_cast<char*>(lock_tables), tid, kTinyThreads);
+  } else {
     const uint4* g = reinterpret_cast<const uint4*>(blob);
     uint4* s = reinterpret_cast<uint4*>(lock_tables);
     for (int i = tid; i < blob_bytes / 16; i += kTinyThreads) s[i] = g[i];
@@ -190,7 +192,7 @@ __device__ __forceinline__ void element_span(const SpanArgs* a) {
 // has one round only.
 template <typename T, bool CLUSTER, typename Shape>
 __global__ void __launch_bounds__(Shape::kThreads, Shape::kPerSm)
-lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem, IoTable io, int op, float scale) {
+lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem, FlatSpec flat, IoTable io, int op, float scale) {
   extern __shared__ __align__(16) unsigned char lock_tables[];
   __shared__ SpanArgs s_span;
   __shared__ char* s_dst[kLockMaxDst];
@@ -202,7 +204,10 @@ lock_kernel(World w, const char* __restrict__ blob, int blob_bytes, int in_smem,
   __syncthreads();
   if (tid < w.P && ld_volatile_u32(&w.ctrl[tid]->abort)) s_ok = 0;
   const char* tab = blob;
-  if (in_smem) {      // one latency for the whole schedule instead of a chain of dependent loads a round
+  if (flat.coll >= 0) {
+    flat_write(flat, w.P, reinterpret_cast<char*>(lock_tables), tid, Shape::kThreads);
+    tab = reinterpret_cast<const char*>(lock_tables);
+  } else if (in_smem) {      // one latency for the whole schedule instead of a chain of dependent loads a round
     const uint4* g = reinterpret_cast<const uint4*>(blob);
     uint4* s = reinterpret_cast<uint4*>(lock_tables);
     for (int i = tid; i < blob_bytes / 16; i += Shape::kThreads) s[i] = g[i];
@@ -334,24 +339,26 @@ extern "C" {
 // each other), the steps fit the span arguments, and no rank's output overlaps any input or another output except as
 // the schedule knows it: the same buffer of one rank (in place), or `slot_bytes` > 0: an input that already lies in its
 // slot of its own output (allgather).
-int chb_lockstep_ok(const chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out, long long slot_bytes) {
-  const Program& g = p->prog;
-  if (c->nlocal != c->P || c->P < 2 || c->trace || g.stats.max_nsrc > kMaxSrc) return 0;
-  const size_t esz = (size_t)dtype_size(dtype);
-  const size_t ni = (size_t)g.in_elems * esz, no = (size_t)g.out_elems * esz;
+static bool lock_buffers_ok(const chb_comm* c, size_t ni, size_t no, bool in_place, const void* const* in, void* const* out, long long slot_bytes) {
+  if (c->nlocal != c->P || c->P < 2 || c->trace) return false;
   for (int b = 0; b < c->P; ++b) {
     const char* o = (const char*)out[b];
     for (int a = 0; a < c->P; ++a) {
       const char* i = (const char*)in[a];
       if (i < o + no && o < i + ni) {
-        const bool known = a == b && ((g.in_place && i == o) || (slot_bytes > 0 && i == o + (size_t)slot_bytes * (size_t)a));
-        if (!known) return 0;
+        const bool known = a == b && ((in_place && i == o) || (slot_bytes > 0 && i == o + (size_t)slot_bytes * (size_t)a));
+        if (!known) return false;
       }
       const char* q = (const char*)out[a];
-      if (a != b && q < o + no && o < q + no) return 0;
+      if (a != b && q < o + no && o < q + no) return false;
     }
   }
-  return 1;
+  return true;
+}
+int chb_lockstep_ok(const chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out, long long slot_bytes) {
+  const Program& g = p->prog;
+  const size_t esz = (size_t)dtype_size(dtype);
+  return g.stats.max_nsrc <= kMaxSrc && lock_buffers_ok(c, (size_t)g.in_elems * esz, (size_t)g.out_elems * esz, g.in_place, in, out, slot_bytes);
 }
 
 // The lockstep schedule of a program for a stored type: laid out and uploaded once.
@@ -409,25 +416,12 @@ int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, long l
   return b->nrounds < 2 || b->saved_rounds > 0 || b->accesses <= kTinyAccesses * b->nrounds;
 }
 
-// Launch a compiled program with all ranks of an emulated world in one grid.  The conditions, refusals and results are
-// chb_run_program's; nctas is per rank as there (0: the launch takes what the message can use).
-int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int op, const void* const* in,
-                             void* const* out, float scale, int nctas, cudaStream_t stream) {
-  if (!c || !p || !in || !out || c->nlocal != c->P) return CHB_ERR_ARG;
-  const Program& g = p->prog;
-  if (g.P != c->P) { c->last_error = "program was compiled for a different number of ranks"; return CHB_ERR_ARG; }
+// One launch for a schedule whose tables are on the device (b.dev) or follow from `flat`.
+static int launch_lockstep(chb_comm* c, const chb_comm::LockBlob& b, const FlatSpec& flat_spec, int dtype, int op, const void* const* in,
+                           void* const* out, float scale, int nctas, cudaStream_t stream) {
   const LockKernels fn = pick_lock(dtype);
-  if (!fn.wide) return CHB_ERR_ARG;
   const size_t esz = (size_t)dtype_size(dtype);
-  if ((size_t)g.work_elems * esz > c->scratch_bytes) {
-    c->last_error = "program needs more symmetric scratch than the communicator has";
-    return CHB_ERR_NO_MEM;
-  }
-  if (op == OP_PROD && dtype == DT_U8) return CHB_ERR_OP;
-  const chb_comm::LockBlob* found = nullptr;
-  const int rc = get_lock_blob(c, p, dtype, &found);
-  if (rc) return rc;
-  const chb_comm::LockBlob& b = *found;
+  FlatSpec flat = flat_spec;
   IoTable io{};
   for (int l = 0; l < c->P; ++l) { io.in[l] = (const char*)in[l]; io.out[l] = (char*)out[l]; }
   long long n = nctas > 0 ? (long long)nctas * c->P : b.max_grains;      // one grain is the least a CTA can be given
@@ -441,14 +435,14 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
   World w = c->world;
   const char* bp = (const char*)b.dev;
   int bytes = b.bytes;
-  int in_smem = b.bytes <= kLockSmemTables && tables_in_smem_wanted() ? 1 : 0;
+  int in_smem = flat.coll >= 0 || (b.bytes <= kLockSmemTables && tables_in_smem_wanted()) ? 1 : 0;
   cudaError_t e;
   const size_t tiny_smem = (size_t)b.bytes + (size_t)b.nrefs * sizeof(void*);
   unsigned long long low = (unsigned long long)b.grid * esz;             // low bits of every address and length
   for (int l = 0; l < c->P; ++l) low |= (unsigned long long)(uintptr_t)in[l] | (unsigned long long)(uintptr_t)out[l];
   const bool vec = (low & 15ull) == 0ull;
-  void* tiny_args[] = {&w, &bp, &bytes, &io, &op, &scale};
-  void* wide_args[] = {&w, &bp, &bytes, &in_smem, &io, &op, &scale};
+  void* tiny_args[] = {&w, &bp, &bytes, &flat, &io, &op, &scale};
+  void* wide_args[] = {&w, &bp, &bytes, &in_smem, &flat, &io, &op, &scale};
   const size_t smem = in_smem ? (size_t)b.bytes : 0;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2] = {};
@@ -485,6 +479,47 @@ int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int o
     return CHB_ERR_CUDA;
   }
   return CHB_SUCCESS;
+}
+
+// Launch a compiled program with all ranks of an emulated world in one grid.  The conditions, refusals and results are
+// chb_run_program's; nctas is per rank as there (0: the launch takes what the message can use).
+int chb_run_program_lockstep(chb_comm* c, const chb_program* p, int dtype, int op, const void* const* in,
+                             void* const* out, float scale, int nctas, cudaStream_t stream) {
+  if (!c || !p || !in || !out || c->nlocal != c->P) return CHB_ERR_ARG;
+  const Program& g = p->prog;
+  if (g.P != c->P) { c->last_error = "program was compiled for a different number of ranks"; return CHB_ERR_ARG; }
+  if (!pick_lock(dtype).wide) return CHB_ERR_ARG;
+  if ((size_t)g.work_elems * (size_t)dtype_size(dtype) > c->scratch_bytes) {
+    c->last_error = "program needs more symmetric scratch than the communicator has";
+    return CHB_ERR_NO_MEM;
+  }
+  if (op == OP_PROD && dtype == DT_U8) return CHB_ERR_OP;
+  const chb_comm::LockBlob* found = nullptr;
+  const int rc = get_lock_blob(c, p, dtype, &found);
+  if (rc) return rc;
+  return launch_lockstep(c, *found, FlatSpec{-1, 0, 0}, dtype, op, in, out, scale, nctas, stream);
+}
+
+// The flat schedule of an allreduce (coll 0), reduce-scatter (1) or allgather (2) of n elements (of a block), which needs no program and keeps
+// nothing: the first call of a length is captured like any other, and costs 55 us where one that compiles and uploads a schedule
+// costs 77 (8 ranks, allreduce of 32 KB, until the result is there; repeated 46).
+// CHB_ERR_UNSUPPORTED, and nothing launched, where the buffers or the type are not lockstep's.
+int chb_run_flat_lockstep(chb_comm* c, int coll, int dtype, int op, const void* const* in, void* const* out, long long n,
+                          float scale, cudaStream_t stream) {
+  const long long esz = dtype_size(dtype);
+  const size_t ni = (size_t)(n * esz) * (coll == 1 ? c->P : 1), no = (size_t)(n * esz) * (coll == 2 ? c->P : 1);
+  if (!pick_lock(dtype).wide || !lock_buffers_ok(c, ni, no, false, in, out, coll == 2 ? n * esz : 0)) return CHB_ERR_UNSUPPORTED;
+  const FlatSpec flat{coll, 0, n};
+  const long long steps = flat_steps(flat.coll, c->P), grains = (n + kLockGrain - 1) / kLockGrain;
+  chb_comm::LockBlob b;
+  b.bytes = flat_bytes(flat.coll, c->P);
+  b.nrefs = flat_refs(flat.coll, c->P);
+  b.nrounds = 1;
+  b.max_grains = steps * grains;
+  b.max_cost = grains * b.nrefs;
+  b.accesses = n * b.nrefs;
+  b.grid = n;                                            // (the offsets are multiples of it)
+  return launch_lockstep(c, b, flat, dtype, op, in, out, scale, 0, stream);
 }
 
 }  // extern "C"

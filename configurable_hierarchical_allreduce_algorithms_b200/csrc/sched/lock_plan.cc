@@ -377,10 +377,7 @@ int simulate_lock_t(const Program& p, const LockPlan& plan, int rop, void* const
   return 0;
 }
 
-}  // namespace
-
-int simulate_lock(const Program& p, int dtype, int op, void* const* in, void* const* out, uint64_t seed, int rewrite, std::string* err) {
-  const LockPlan plan = make_lock_plan(p, rewrite);
+int simulate_plan(const Program& p, const LockPlan& plan, int dtype, int op, void* const* in, void* const* out, uint64_t seed, std::string* err) {
   switch (dtype) {
     case DT_F32: return simulate_lock_t<float>(p, plan, op, in, out, seed, err);
     case DT_F64: return simulate_lock_t<double>(p, plan, op, in, out, seed, err);
@@ -390,6 +387,44 @@ int simulate_lock(const Program& p, int dtype, int op, void* const* in, void* co
   }
   if (err) *err = "simulate: unsupported dtype on the host";
   return -2;
+}
+
+}  // namespace
+
+int simulate_lock(const Program& p, int dtype, int op, void* const* in, void* const* out, uint64_t seed, int rewrite, std::string* err) {
+  return simulate_plan(p, make_lock_plan(p, rewrite), dtype, op, in, out, seed, err);
+}
+
+int simulate_flat(const FlatSpec& f, int P, int dtype, int op, void* const* in, void* const* out, uint64_t seed, std::string* err) {
+  std::vector<char> table((size_t)flat_bytes(f.coll, P), (char)0xEE);
+  const int stride = 1 + (int)(seed % 7);
+  for (int first = stride - 1; first >= 0; --first) flat_write(f, P, table.data(), first, stride);
+  const LockHeader* h = reinterpret_cast<const LockHeader*>(table.data());
+  const LockRound* rounds = reinterpret_cast<const LockRound*>(h + 1);
+  const LockStep* steps = reinterpret_cast<const LockStep*>(rounds + h->nrounds);
+  const LockRef* refs = reinterpret_cast<const LockRef*>(steps + h->nsteps);
+  LockPlan plan;
+  plan.P = P;
+  plan.nrounds = h->nrounds;
+  for (int i = rounds[0].step_begin; i < rounds[0].step_end; ++i) {
+    LockStepPlan x;
+    x.count = steps[i].count;
+    x.final = steps[i].final != 0;
+    const LockRef* r = refs + steps[i].ref_begin;
+    for (int q = 0; q < steps[i].nsrc; ++q) x.srcs.push_back(Src{r[q].rank, r[q].buf, r[q].off});
+    for (int q = 0; q < steps[i].ndst; ++q) x.dsts.push_back(LockDst{r[steps[i].nsrc + q].rank, r[steps[i].nsrc + q].buf, r[steps[i].nsrc + q].off});
+    plan.steps.push_back(x);
+  }
+  // the places of steps and costs are those that the tables of such a plan have
+  const std::vector<char> built = make_lock_blob(plan);
+  if (built.size() != table.size() || std::memcmp(built.data(), table.data(), table.size()) != 0) {
+    if (err) *err = "the flat schedule's table is not that of its steps";
+    return -1;
+  }
+  Program p;
+  p.P = P;
+  p.name = "flat";
+  return simulate_plan(p, plan, dtype, op, in, out, seed, err);
 }
 
 }  // namespace chb

@@ -92,9 +92,48 @@ struct LockRef { long long off; int rank, buf; };
 static_assert(sizeof(LockHeader) % 16 == 0 && sizeof(LockRound) % 16 == 0 && sizeof(LockStep) % 16 == 0 && sizeof(LockRef) % 16 == 0, "copied as 16-byte words");
 std::vector<char> make_lock_blob(const LockPlan& p);
 
+// What the one-shot and two-shot line kernels compute, in these tables: operands in rank order, every rank the same result.
+// One round: an allreduce is one step (all inputs, all outputs), a reduce-scatter and an allgather one step per block.  It
+// follows from a few numbers, so a CTA writes it into its shared memory (entries first, first + stride, ...) instead of
+// reading it from a table that somebody has to allocate and upload: the call needs nothing that lasts.
+struct FlatSpec { int coll, pad; long long n; };       // coll: 0 allreduce, 1 reduce-scatter, 2 allgather, -1 none; n: elements (of a block)
+CHB_HOST_DEVICE inline int flat_steps(int coll, int P) { return coll == 0 ? 1 : P; }
+CHB_HOST_DEVICE inline int flat_nsrc(int coll, int P) { return coll == 2 ? 1 : P; }
+CHB_HOST_DEVICE inline int flat_ndst(int coll, int P) { return coll == 1 ? 1 : P; }
+CHB_HOST_DEVICE inline int flat_refs(int coll, int P) { return flat_steps(coll, P) * (flat_nsrc(coll, P) + flat_ndst(coll, P)); }
+CHB_HOST_DEVICE inline int flat_bytes(int coll, int P) {
+  return (int)(sizeof(LockHeader) + sizeof(LockRound)) + flat_steps(coll, P) * (int)sizeof(LockStep) + flat_refs(coll, P) * (int)sizeof(LockRef);
+}
+CHB_HOST_DEVICE inline void flat_write(const FlatSpec& f, int P, char* table, int first, int stride) {
+  LockHeader* h = reinterpret_cast<LockHeader*>(table);
+  LockRound* round = reinterpret_cast<LockRound*>(h + 1);
+  LockStep* steps = reinterpret_cast<LockStep*>(round + 1);
+  const int nsteps = flat_steps(f.coll, P), nsrc = flat_nsrc(f.coll, P), refs_per = nsrc + flat_ndst(f.coll, P);
+  LockRef* refs = reinterpret_cast<LockRef*>(steps + nsteps);
+  const long long cost = (f.n + kLockGrain - 1) / kLockGrain * refs_per;
+  for (int i = first; i < nsteps * refs_per + nsteps + 1; i += stride) {
+    if (i < nsteps * refs_per) {
+      const int s = i / refs_per, q = i % refs_per;      // the q-th reference of block s
+      LockRef r;
+      r.buf = q < nsrc ? P_IN : P_OUT;
+      if (q < nsrc) { r.rank = f.coll == 2 ? s : q; r.off = f.coll == 1 ? s * f.n : 0; }
+      else { r.rank = f.coll == 1 ? s : q - nsrc; r.off = f.coll == 2 ? s * f.n : 0; }
+      refs[i] = r;
+    } else if (i < nsteps * refs_per + nsteps) {
+      const int s = i - nsteps * refs_per;
+      steps[s] = LockStep{s * cost, f.n, s * f.n, s * refs_per, nsrc, refs_per - nsrc, f.coll == 2 ? 0 : 1, 0, 0};
+    } else {
+      *h = LockHeader{1, nsteps, nsteps * refs_per, 0};
+      *round = LockRound{0, nsteps, nsteps * cost, nsteps * f.n, 0};
+    }
+  }
+}
+
 // Executes the plan on host memory, the steps of a round in random order and the destinations of a step as lock_passes
 // has them stored at these addresses, and checks that no step of a round touches what another one writes.  Returns 0, -1 (err says what) or -2 for a bad argument.
 int simulate_lock(const Program& p, int dtype, int op, void* const* in, void* const* out, uint64_t seed,
                   int rewrite, std::string* err);
+// The same for the flat schedule, as flat_write lays it out.
+int simulate_flat(const FlatSpec& f, int P, int dtype, int op, void* const* in, void* const* out, uint64_t seed, std::string* err);
 
 }  // namespace chb

@@ -200,6 +200,21 @@ class Program:
             raise RuntimeError(f"simulate_lock({self.name}) failed: {err.value.decode()}")
         return [o[:self.out_elems] for o in outs]
 
+    @staticmethod
+    def simulate_flat(coll: str, inputs: list[np.ndarray], op: str = "sum", seed: int = 0) -> list[np.ndarray]:
+        """The flat lockstep schedule (operands in rank order, one round; it has no program) on host arrays."""
+        P, n = len(inputs), inputs[0].size // (len(inputs) if coll == "reduce_scatter" else 1)
+        dt = np.dtype(inputs[0].dtype)
+        ins = [np.ascontiguousarray(x) for x in inputs]
+        outs = [np.zeros(n * (P if coll == "allgather" else 1), dtype=dt) for _ in range(P)]
+        err = C.create_string_buffer(512)
+        rc = N.lib().chb_simulate_flat({"allreduce": 0, "reduce_scatter": 1, "allgather": 2}[coll], P, _DT_FROM_NP[dt], _OPS[op],
+                                       (C.c_void_p * P)(*[x.ctypes.data for x in ins]),
+                                       (C.c_void_p * P)(*[x.ctypes.data for x in outs]), n, seed, err, len(err))
+        if rc:
+            raise RuntimeError(f"simulate_flat({coll}) failed: {err.value.decode()}")
+        return outs
+
     def lock_info(self, rewrite: int = 2) -> dict:
         """Rounds, steps, elements read and elements stored of the lockstep form."""
         v = (C.c_longlong * 4)()

@@ -220,3 +220,35 @@ def test_skewed_destinations_around_the_longest_element_wise_span(cuda, coll):
                 assert not full[r][:r].any() and not full[r][r + n_out:].any()
     comm.check()
     comm.close()
+
+
+def test_first_call_of_a_length_may_be_captured(cuda):
+    """Automatic small calls need no schedule that lasts: the first call of a new length is captured, and its replay
+    survives more other lengths than the program cache holds."""
+    P, n = 8, 3001
+    comm = Communicator.emulated(P, ll_bytes=1 << 20, scratch_bytes=8 << 20, user_bytes=4096)
+    src = [torch.randn(n * P, device="cuda") for _ in range(P)]
+    blocks = [s[:n].clone() for s in src]
+    ar, rs = [torch.zeros(n, device="cuda") for _ in range(P)], [torch.zeros(n, device="cuda") for _ in range(P)]
+    ag = [torch.zeros(n * P, device="cuda") for _ in range(P)]
+
+    def calls(m):
+        chb.all_reduce(comm, [b[:m] for b in blocks], out=[x[:m] for x in ar])
+        chb.reduce_scatter(comm, [s[:m * P] for s in src], out=[x[:m] for x in rs])
+        chb.all_gather(comm, [b[:m] for b in blocks], out=[x[:m * P] for x in ag])
+
+    calls(n - 1)                                            # (loads the kernels)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        calls(n)
+    for m in range(16, 1516):                               # (the smallest ones belong to another row of the tuned table)
+        calls(m)
+    for x in ar + rs + ag:
+        x.zero_()
+    graph.replay()
+    full = chb.all_reduce(comm, src, algo="ll")             # operands in rank order, as here
+    for r in range(P):
+        assert torch.equal(ar[r], full[0][:n]) and torch.equal(rs[r], full[0][r * n:(r + 1) * n])
+        assert torch.equal(ag[r], torch.cat(blocks))
+    comm.check()
+    comm.close()

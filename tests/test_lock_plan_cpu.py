@@ -76,3 +76,23 @@ def test_in_place_on_different_16_byte_grids(algo, dtype):
                         assert got[r].tobytes() == want[r].tobytes(), (P, k, b, low, skew, rewrite, r)
                 several += 1
     assert several
+
+
+@pytest.mark.parametrize("P", [2, 3, 8, 16])
+def test_flat_schedule_without_a_program(P):
+    """The tables that a CTA writes for itself: the entries and costs of the plan they describe, and the line kernels'
+    result (operands in rank order), around a grain of 2048 elements."""
+    rng = np.random.default_rng(P)
+    for n in (1, 7, 2047, 2048, 2049, 5001):
+        xs = [rng.standard_normal(n * P).astype(np.float32) for _ in range(P)]
+        total = xs[0].copy()
+        for x in xs[1:]:
+            total = total + x
+        for seed in (0, 5):
+            for got in chb.Program.simulate_flat("allreduce", xs, seed=seed):
+                assert got.tobytes() == total.tobytes()
+            for r, got in enumerate(chb.Program.simulate_flat("reduce_scatter", xs, seed=seed)):
+                assert got.tobytes() == total[r * n:(r + 1) * n].tobytes()
+            blocks = [x[:n].copy() for x in xs]
+            for got in chb.Program.simulate_flat("allgather", blocks, seed=seed):
+                assert got.tobytes() == np.concatenate(blocks).tobytes()
