@@ -209,7 +209,9 @@ __device__ __forceinline__ bool cta_barrier(const World& w, Ctrl* c, int rank, u
 // ------------------------------------------------------------------ overlapped launches
 // A kernel that is usually launched right behind another one starts with dependent_launch(): its CTAs may be placed while
 // the grid before it in the stream drains (launch_overlapped), and wait here until that grid has completed and its writes
-// are visible.  Nothing of global memory may be touched before.
+// are visible.  Nothing of global memory may be touched before, and no data pointer may be `const __restrict__`: the
+// compiler may read through such a pointer on the read-only path, whose contract is that nobody writes there while the
+// kernel lives, which here includes the end of the kernel that produces the data.
 __device__ __forceinline__ void dependent_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -164,12 +164,13 @@ rs_adam_local_kernel(World w, AdamIo io, long long n, AdamHyper h) {
 // already been allreduced; AdamW on the fp32 master, bf16 copy of the result.
 // Bound by HBM (30 bytes an element); one vector a thread, short CTAs, as above.
 __global__ void __launch_bounds__(kLocalAdamThreads)
-adam_flat_kernel(const float* __restrict__ grad, float* master, float* m, float* v, __nv_bfloat16* param,
+adam_flat_kernel(const float* grad, float* master, float* m, float* v, __nv_bfloat16* param,
                  long long n, AdamHyper h) {
   const long long i = (long long)blockIdx.x * kLocalAdamThreads + threadIdx.x;
   dependent_launch();
   if (i >= n / 4) return;
-  const float4 g = reinterpret_cast<const float4*>(grad)[i];
+  const uint4 loaded = ld16_cg(grad + i * 4);
+  const float4 g = *reinterpret_cast<const float4*>(&loaded);
   float4 ww = reinterpret_cast<float4*>(master)[i], m1 = reinterpret_cast<float4*>(m)[i], v1 = reinterpret_cast<float4*>(v)[i];
   const float s = h.grad_scale;
   __nv_bfloat16 o[4];

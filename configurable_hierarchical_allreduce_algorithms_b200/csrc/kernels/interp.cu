@@ -451,7 +451,7 @@ constexpr int kCopyCtasPerSm = 16;   // two waves of eight resident CTAs: measur
 
 // nvec: number of 32-byte vectors; src / dst 32-byte aligned.
 __global__ void __launch_bounds__(kCopyThreads)
-local_copy_kernel(Ctrl* c, const char* __restrict__ src, char* __restrict__ dst, long long nvec, int nrounds) {
+local_copy_kernel(Ctrl* c, const char* src, char* dst, long long nvec, int nrounds) {
   dependent_launch();
   const long long tile = (long long)kCopyThreads * kCopyUnroll;
   const long long ntiles = (nvec + tile - 1) / tile;
