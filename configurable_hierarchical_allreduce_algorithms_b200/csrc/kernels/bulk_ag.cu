@@ -173,37 +173,44 @@ ag_bulk_kernel(World w, BulkIo io, long long nbytes) {
 constexpr int kLocalThreads = 256, kLocalUnroll = 4;
 
 // WIDE: 32-byte vectors (every pointer and the block length a multiple of 32), else 16-byte ones.
-template <bool WIDE>
+// LIMITED: the caller gave a number of CTAs (of 256 threads, for each rank), which take the pieces in turn.
+template <bool WIDE, bool LIMITED>
 __global__ void __launch_bounds__(kLocalThreads)
 ag_local_kernel(World w, BulkIo io, long long nbytes) {
   constexpr int V = WIDE ? 32 : 16;
   const int P = w.P, owner = (int)blockIdx.y;
   dependent_launch();
   const unsigned aborted = (int)threadIdx.x < P ? ld_volatile_u32(&w.ctrl[threadIdx.x]->abort) : 0u;   // (travels with the data)
-  const long long nv = nbytes / V, j0 = (long long)blockIdx.x * (kLocalThreads * kLocalUnroll) + threadIdx.x;
+  if (LIMITED && __syncthreads_or((int)aborted)) return;
+  constexpr int kPiece = kLocalThreads * kLocalUnroll;
+  const long long nv = nbytes / V;
   const char* src = io.in[owner];
-  uint4 lo[kLocalUnroll], hi[kLocalUnroll];
-#pragma unroll
-  for (int u = 0; u < kLocalUnroll; ++u) {
-    const long long j = j0 + u * kLocalThreads;
-    lo[u] = hi[u] = make_uint4(0u, 0u, 0u, 0u);
-    if (j < nv) {
-      if (WIDE) ld32_cg(src + j * V, lo[u], hi[u]);
-      else lo[u] = ld16_cg(src + j * V);
-    }
-  }
-  if (__syncthreads_or((int)aborted)) return;
-  for (int i = 0; i < P; ++i) {
-    char* dst = io.out[i] + (long long)owner * nbytes;
-    if (dst == src) continue;                      // (a block that already lies in its slot)
+  for (long long piece = blockIdx.x; piece * kPiece < nv; piece += gridDim.x) {
+    const long long j0 = piece * kPiece + threadIdx.x;
+    uint4 lo[kLocalUnroll], hi[kLocalUnroll];
 #pragma unroll
     for (int u = 0; u < kLocalUnroll; ++u) {
       const long long j = j0 + u * kLocalThreads;
+      lo[u] = hi[u] = make_uint4(0u, 0u, 0u, 0u);
       if (j < nv) {
-        if (WIDE) st32(dst + j * V, lo[u], hi[u]);
-        else st16(dst + j * V, lo[u]);
+        if (WIDE) ld32_cg(src + j * V, lo[u], hi[u]);
+        else lo[u] = ld16_cg(src + j * V);
       }
     }
+    if (!LIMITED && __syncthreads_or((int)aborted)) return;
+    for (int i = 0; i < P; ++i) {
+      char* dst = io.out[i] + (long long)owner * nbytes;
+      if (dst == src) continue;                      // (a block that already lies in its slot)
+#pragma unroll
+      for (int u = 0; u < kLocalUnroll; ++u) {
+        const long long j = j0 + u * kLocalThreads;
+        if (j < nv) {
+          if (WIDE) st32(dst + j * V, lo[u], hi[u]);
+          else st16(dst + j * V, lo[u]);
+        }
+      }
+    }
+    if (!LIMITED) break;
   }
   // (no wait can expire here, so the launch counters need no order with the copies)
   if (blockIdx.x == 0 && owner == 0 && (int)threadIdx.x < P) w.ctrl[threadIdx.x]->status[6] += 1ull;
@@ -261,8 +268,11 @@ int chb_ag_bulk(chb_comm* c, const void* const* in, void* const* out, long long 
     for (int l = 0; l < c->P; ++l) low |= (unsigned long long)(uintptr_t)in[l] | (unsigned long long)(uintptr_t)out[l];
     const bool wide = (low & 31ull) == 0ull;
     const long long piece = (long long)kLocalThreads * kLocalUnroll * (wide ? 32 : 16);
-    const dim3 grid((unsigned)((nbytes + piece - 1) / piece), (unsigned)c->P, 1);
-    const cudaError_t e = launch_overlapped(wide ? ag_local_kernel<true> : ag_local_kernel<false>, grid, dim3(kLocalThreads), stream, c->world, io, nbytes);
+    const long long pieces = (nbytes + piece - 1) / piece;
+    const bool limited = nctas > 0 && pieces > nctas;
+    const dim3 grid((unsigned)(limited ? nctas : pieces), (unsigned)c->P, 1);
+    const cudaError_t e = launch_overlapped(limited ? (wide ? ag_local_kernel<true, true> : ag_local_kernel<false, true>)
+                                                    : (wide ? ag_local_kernel<true, false> : ag_local_kernel<false, false>), grid, dim3(kLocalThreads), stream, c->world, io, nbytes);
     if (e != cudaSuccess) { c->last_error = "bulk allgather launch failed"; return CHB_ERR_CUDA; }
     return CHB_SUCCESS;
   }

@@ -113,49 +113,56 @@ rs_adam_kernel(World w, AdamIo io, long long n, AdamHyper h, const char* mc_grad
 // of the parameters, 1.2 GB in all).
 constexpr int kLocalAdamThreads = 256;
 
+// LIMITED: the caller gave a number of CTAs (of 256 threads, for each rank), which take the vectors in turn.
+template <bool LIMITED>
 __global__ void __launch_bounds__(kLocalAdamThreads, 4)
 rs_adam_local_kernel(World w, AdamIo io, long long n, AdamHyper h) {
   const int P = w.P, rank = (int)blockIdx.y;
   dependent_launch();
   const unsigned aborted = (int)threadIdx.x < P ? ld_volatile_u32(&w.ctrl[threadIdx.x]->abort) : 0u;   // (travels with the data)
-  const long long nvec = n / 4, i = (long long)blockIdx.x * kLocalAdamThreads + threadIdx.x;
-  const bool live = i < nvec;
-  const long long at = (long long)rank * nvec + i;
-  float4 ww = make_float4(0.f, 0.f, 0.f, 0.f), m1 = ww, v1 = ww, g = ww;
-  if (live) {
-    ww = reinterpret_cast<const float4*>(io.master[rank])[i];
-    m1 = reinterpret_cast<const float4*>(io.m[rank])[i];
-    v1 = reinterpret_cast<const float4*>(io.v[rank])[i];
-  }
-  constexpr int G = 8;
-#pragma unroll 1
-  for (int q0 = 0; q0 < P; q0 += G) {
-    uint4 t[G];
-#pragma unroll
-    for (int q = 0; q < G; ++q) {
-      t[q] = make_uint4(0u, 0u, 0u, 0u);
-      if (live && q0 + q < P) t[q] = ld16_cg(reinterpret_cast<const char*>(io.grad[q0 + q]) + at * 16);
+  if (LIMITED && __syncthreads_or((int)aborted)) return;
+  const long long nvec = n / 4;
+  for (long long i = (long long)blockIdx.x * kLocalAdamThreads + threadIdx.x;; i += (long long)gridDim.x * kLocalAdamThreads) {
+    const bool live = i < nvec;
+    if (LIMITED && !live) break;
+    const long long at = (long long)rank * nvec + i;
+    float4 ww = make_float4(0.f, 0.f, 0.f, 0.f), m1 = ww, v1 = ww, g = ww;
+    if (live) {
+      ww = reinterpret_cast<const float4*>(io.master[rank])[i];
+      m1 = reinterpret_cast<const float4*>(io.m[rank])[i];
+      v1 = reinterpret_cast<const float4*>(io.v[rank])[i];
     }
+    constexpr int G = 8;
+#pragma unroll 1
+    for (int q0 = 0; q0 < P; q0 += G) {
+      uint4 t[G];
 #pragma unroll
-    for (int q = 0; q < G; ++q) {      // rank order: identical bits on every run
-      if (q0 + q < P) {
-        const float4 x = *reinterpret_cast<const float4*>(&t[q]);
-        g.x += x.x; g.y += x.y; g.z += x.z; g.w += x.w;
+      for (int q = 0; q < G; ++q) {
+        t[q] = make_uint4(0u, 0u, 0u, 0u);
+        if (live && q0 + q < P) t[q] = ld16_cg(reinterpret_cast<const char*>(io.grad[q0 + q]) + at * 16);
+      }
+#pragma unroll
+      for (int q = 0; q < G; ++q) {      // rank order: identical bits on every run
+        if (q0 + q < P) {
+          const float4 x = *reinterpret_cast<const float4*>(&t[q]);
+          g.x += x.x; g.y += x.y; g.z += x.z; g.w += x.w;
+        }
       }
     }
-  }
-  if (__syncthreads_or((int)aborted)) return;
-  if (live) {
-    const float s = h.grad_scale;
-    __nv_bfloat16 o[4];
-    o[0] = __float2bfloat16_rn(adam_one(g.x * s, ww.x, m1.x, v1.x, h));
-    o[1] = __float2bfloat16_rn(adam_one(g.y * s, ww.y, m1.y, v1.y, h));
-    o[2] = __float2bfloat16_rn(adam_one(g.z * s, ww.z, m1.z, v1.z, h));
-    o[3] = __float2bfloat16_rn(adam_one(g.w * s, ww.w, m1.w, v1.w, h));
-    reinterpret_cast<float4*>(io.master[rank])[i] = ww;
-    reinterpret_cast<float4*>(io.m[rank])[i] = m1;
-    reinterpret_cast<float4*>(io.v[rank])[i] = v1;
-    reinterpret_cast<uint2*>(io.param[rank])[i] = *reinterpret_cast<uint2*>(o);
+    if (!LIMITED && __syncthreads_or((int)aborted)) return;
+    if (live) {
+      const float s = h.grad_scale;
+      __nv_bfloat16 o[4];
+      o[0] = __float2bfloat16_rn(adam_one(g.x * s, ww.x, m1.x, v1.x, h));
+      o[1] = __float2bfloat16_rn(adam_one(g.y * s, ww.y, m1.y, v1.y, h));
+      o[2] = __float2bfloat16_rn(adam_one(g.z * s, ww.z, m1.z, v1.z, h));
+      o[3] = __float2bfloat16_rn(adam_one(g.w * s, ww.w, m1.w, v1.w, h));
+      reinterpret_cast<float4*>(io.master[rank])[i] = ww;
+      reinterpret_cast<float4*>(io.m[rank])[i] = m1;
+      reinterpret_cast<float4*>(io.v[rank])[i] = v1;
+      reinterpret_cast<uint2*>(io.param[rank])[i] = *reinterpret_cast<uint2*>(o);
+    }
+    if (!LIMITED) break;
   }
   if (blockIdx.x == 0 && rank == 0 && (int)threadIdx.x < P) w.ctrl[threadIdx.x]->status[6] += 1ull;
 }
@@ -230,8 +237,10 @@ int chb_rs_adam(chb_comm* c, const void* const* grad, void* const* master, void*
   if (n == 0) return CHB_SUCCESS;
   AdamHyper h{hyper[0], hyper[1], hyper[2], hyper[3], hyper[4], hyper[5], hyper[6], hyper[7]};
   if (c->nlocal == c->P && !c->trace && !mc) {
-    const dim3 grid((unsigned)((n / 4 + kLocalAdamThreads - 1) / kLocalAdamThreads), (unsigned)c->P, 1);
-    if (launch_overlapped(rs_adam_local_kernel, grid, dim3(kLocalAdamThreads), stream, c->world, io, n, h) != cudaSuccess) { c->last_error = "rs_adam launch failed"; return CHB_ERR_CUDA; }
+    const long long ctas = (n / 4 + kLocalAdamThreads - 1) / kLocalAdamThreads;
+    const bool limited = nctas > 0 && ctas > nctas;
+    const dim3 grid((unsigned)(limited ? nctas : ctas), (unsigned)c->P, 1);
+    if (launch_overlapped(limited ? rs_adam_local_kernel<true> : rs_adam_local_kernel<false>, grid, dim3(kLocalAdamThreads), stream, c->world, io, n, h) != cudaSuccess) { c->last_error = "rs_adam launch failed"; return CHB_ERR_CUDA; }
     return CHB_SUCCESS;
   }
   const int max_pair_ctas = (kSigSlots - kSigNvlsBase) / kMaxRanks;

@@ -106,7 +106,7 @@ def _run_local(comm: Communicator, coll: str, ins, outs, count: int, op, scale, 
 def _run(comm: Communicator, coll: str, ins, outs, count: int, op, algo, k, b, aux, scale, nctas, stream,
          payload_bytes: int, ll_mode: int):
     """Pick the kernel and enqueue it with a single native call."""
-    auto = algo == "auto"
+    auto, given = algo == "auto", nctas
     if auto and comm.nlocal > 1 and nctas == 0 and not _NVTX:
         if _run_local(comm, coll, ins, outs, count, op, scale, stream, payload_bytes):
             return
@@ -127,6 +127,8 @@ def _run(comm: Communicator, coll: str, ins, outs, count: int, op, algo, k, b, a
         elif algo.startswith("nvls") and not (comm.has_multicast and sym and comm.nlocal == 1
                                               and payload_bytes % 16 == 0):
             algo, k, b = "radix_batch", 2, 1
+        if comm.nlocal > 1 and algo == "bulk":
+            nctas = given                       # (the table's CTAs were measured with one rank per GPU)
         if comm.nlocal > 1 and algo.startswith("radix_batch:"):
             algo = "radix_batch"                # mode and CTAs were measured with one rank per GPU
             nctas = 0 if nctas == choice.nctas else nctas
