@@ -127,11 +127,9 @@ def _run(comm: Communicator, coll: str, ins, outs, count: int, op, algo, k, b, a
         elif algo.startswith("nvls") and not (comm.has_multicast and sym and comm.nlocal == 1
                                               and payload_bytes % 16 == 0):
             algo, k, b = "radix_batch", 2, 1
-        if comm.nlocal > 1 and algo == "bulk":
-            nctas = given                       # (the table's CTAs were measured with one rank per GPU)
-        if comm.nlocal > 1 and algo.startswith("radix_batch:"):
-            algo = "radix_batch"                # mode and CTAs were measured with one rank per GPU
-            nctas = 0 if nctas == choice.nctas else nctas
+        if comm.nlocal > 1 and (algo == "bulk" or algo.startswith("radix_batch:")):
+            algo = algo.split(":")[0]           # mode and CTAs were measured with one rank per GPU
+            nctas = given
         if coll == "allreduce" and count % comm.P:
             algo, k, b = any_count(coll, algo, k, b, count, comm.P, _ll_ok(comm, ins, outs, payload_bytes), payload_bytes)
     if algo == "bulk" and not (coll == "allgather" and payload_bytes % 16 == 0 and comm.is_symmetric(ins[0])

@@ -123,3 +123,23 @@ def test_the_sizes_of_the_benchmark_sweep_reach_a_kernel_that_takes_them(P, mult
     # the tuned hierarchical cell is still used where the length allows it (8 ranks: the 32-byte vector of the sweep)
     if P == 8 and multicast:
         assert any(name.startswith("radix_batch:ll") and coll == 0 and b == P for coll, name, k, b, count in fake.calls)
+
+
+@pytest.mark.parametrize("row", [("radix_batch:ll", 2, 1, 128), ("radix_batch:pull", 2, 1, 64), ("bulk", 2, 1, 64)])
+@pytest.mark.parametrize("nctas", [0, 1, 64, 128])
+def test_an_emulated_world_keeps_the_callers_ctas_and_drops_the_tables(row, nctas, monkeypatch):
+    """The table's CTAs belong to one rank per GPU; a number that the caller gives stands, also where it is the table's."""
+    from configurable_hierarchical_allreduce_algorithms_b200 import _native as N
+    from configurable_hierarchical_allreduce_algorithms_b200.ops import collectives as ops
+
+    calls = []
+    fake = SimpleNamespace(chb_collective=lambda *a: calls.append((a[2].decode(), a[12])) or 0)
+    monkeypatch.setattr(N, "lib", lambda: fake)
+    monkeypatch.setattr(ops, "_stream_ptr", lambda s: None)
+    monkeypatch.setattr(ops, "_run_local", lambda *a: False)
+    monkeypatch.setattr(autotune, "choose", lambda *a: autotune.Choice(*row))
+    comm = SimpleNamespace(P=2, nlocal=2, _h=None, _choices={}, launches=0, ll_max_bytes=4 << 20, ll2_max_bytes=4 << 20, has_multicast=False,
+                           is_symmetric=lambda t: True, _err=lambda rc: None)
+    ts = [SimpleNamespace(element_size=lambda: 4, dtype=torch.float32, data_ptr=lambda: 4096) for _ in range(2)]
+    ops._run(comm, "allgather", ts, ts, 1 << 20, "sum", "auto", 2, 1, 0, 1.0, nctas, None, 4 << 20, ops.LL_AG)
+    assert calls == [(row[0].split(":")[0], nctas)]
