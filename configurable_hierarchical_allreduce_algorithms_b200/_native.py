@@ -59,6 +59,8 @@ def _declare(L: C.CDLL) -> None:
     L.chb_program_simulate_ll.argtypes = [vp, i32, i32, C.POINTER(vp), C.POINTER(vp), u64, i32, i32, i32, cp, i32]
     L.chb_program_lock_info.restype = i32
     L.chb_program_lock_info.argtypes = [vp, i32, C.POINTER(C.c_longlong), i32]
+    L.chb_program_lock_preferred.restype = i32
+    L.chb_program_lock_preferred.argtypes = [vp, i32, i32]
     L.chb_program_simulate_lock.restype = i32
     L.chb_program_simulate_lock.argtypes = [vp, i32, i32, C.POINTER(vp), C.POINTER(vp), u64, i32, cp, i32]
     L.chb_simulate_flat.restype = i32

@@ -84,6 +84,9 @@ int chb_program_simulate_ll(const chb_program_t* p, int dtype, int op, void* con
  * chb_program_simulate_lock: run it on host buffers, the steps of a round in a random order (seed); two steps of one
  *   round that touch the same memory end the run with CHB_ERR_TIMEOUT and their round in err. */
 int chb_program_lock_info(const chb_program_t* p, int rewrite, long long* info, int n);
+/* 1: an emulated world runs the program in lockstep where it could also be pushed with flagged lines; on_grid16: every
+ * buffer and length is a multiple of 16 bytes. */
+int chb_program_lock_preferred(const chb_program_t* p, int dtype, int on_grid16);
 int chb_program_simulate_lock(const chb_program_t* p, int dtype, int op, void* const* in, void* const* out,
                               uint64_t seed, int rewrite, char* err, int errlen);
 /* The same for the flat schedule of an allreduce, reduce-scatter or allgather (count as in chb_collective), which has no

@@ -1,4 +1,5 @@
 // C ABI for step programs (chb.h, "programs" section).
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <exception>
@@ -156,6 +157,20 @@ int chb_program_lock_info(const chb_program_t* p, int rewrite, long long* info, 
   const long long v[4] = {plan.nrounds, (long long)plan.steps.size(), reads, stores};
   for (int i = 0; i < n && i < 4; ++i) info[i] = v[i];
   return CHB_SUCCESS;
+}
+
+int chb_program_lock_preferred(const chb_program_t* p, int dtype, int on_grid16) {
+  if (!p) return 0;
+  const chb::LockPlan plan = chb::make_lock_plan(p->prog, chb::lock_rewrite_for(dtype));
+  long long accesses = 0, refs = 0;
+  for (const chb::LockStepPlan& x : plan.steps) {
+    const long long n = (long long)(x.srcs.size() + x.dsts.size());
+    refs += n;
+    accesses += x.count * n;
+  }
+  return chb::lock_beats_push(plan.nrounds, chb::lock_saved_rounds(p->prog, plan), accesses,
+                              chb::lock_blob_bytes(plan.nrounds, (long long)plan.steps.size(), refs), refs,
+                              std::max(p->prog.in_elems, p->prog.out_elems) * (int64_t)chb::dtype_size(dtype), chb::dtype_size(dtype), on_grid16 != 0);
 }
 
 int chb_program_simulate_lock(const chb_program_t* p, int dtype, int op, void* const* in, void* const* out,

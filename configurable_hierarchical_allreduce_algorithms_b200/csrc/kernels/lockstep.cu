@@ -20,6 +20,7 @@
 //
 // The ranks' epochs and signal pads are left alone (nobody is signalled and nobody waits), so launches of this kernel
 // and of the per-rank ones mix freely on one communicator.
+#include <algorithm>
 #include <cstring>
 #include <vector>
 
@@ -33,10 +34,8 @@
 namespace chb {
 
 constexpr int kTinyThreads = 1024;
-constexpr long long kTinyAccesses = 8192;          // loads + stores a round, on average, up to which one CTA runs the schedule
 constexpr int kLockCluster = 8;                    // CTAs of a cluster launch
 constexpr long long kClusterGrains = 32;           // grains of a round up to which a cluster runs the schedule
-constexpr long long kLockSmemTables = 40 << 10;   // schedules up to this size are kept in shared memory
 
 // Barrier over the grid in two halves, so that a CTA works out its share of the next round while the others arrive: one
 // release, one acquire poll, and the abort word only on the slow path.
@@ -386,7 +385,7 @@ static int get_lock_blob(chb_comm* c, const chb_program* p, int dtype, const chb
       b.max_grains = grains > b.max_grains ? grains : b.max_grains;
     }
     b.nrounds = plan.nrounds;
-    b.saved_rounds = make_lock_plan(g, LOCK_PLAIN).nrounds - plan.nrounds;
+    b.saved_rounds = lock_saved_rounds(g, plan);
     const std::vector<char> host = make_lock_blob(plan);
     b.bytes = (int)host.size();
     if (cudaMalloc(&b.dev, host.size()) != cudaSuccess) { c->last_error = "cudaMalloc(lockstep schedule) failed"; return CHB_ERR_NO_MEM; }
@@ -406,14 +405,18 @@ int chb_program_fits(const chb_comm* c, const chb_program* p, int dtype) {
   return (size_t)p->prog.work_elems * (size_t)dtype_size(dtype) <= c->scratch_bytes;
 }
 
-// Small schedules of which the rewriting shortens nothing (recursive doubling, recursive halving: every round is an
-// exchange that reduces) run faster with flagged lines, whose rounds have no barrier: 8 ranks, recursive doubling
-// 40 / 130 / 256 / 512 KB 15.3 / 15.5 / 19.5 / 20.7 us in lockstep, 13.9 / 14.0 / 22.2 / 38.7 us with lines.
-constexpr long long kPushBytes = 192 << 10;
-int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, long long payload_bytes) {
+// Everything on the 16-byte grid: addresses, offsets and lengths.
+static bool lock_on_grid16(const chb_comm* c, const chb_comm::LockBlob& b, size_t esz, const void* const* in, void* const* out) {
+  unsigned long long low = (unsigned long long)b.grid * esz;
+  for (int l = 0; l < c->P; ++l) low |= (unsigned long long)(uintptr_t)in[l] | (unsigned long long)(uintptr_t)out[l];
+  return (low & 15ull) == 0ull;
+}
+int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out) {
   const chb_comm::LockBlob* b = nullptr;
-  if (payload_bytes > kPushBytes || get_lock_blob(c, p, dtype, &b)) return 1;     // (the launch reports what is wrong)
-  return b->nrounds < 2 || b->saved_rounds > 0 || b->accesses <= kTinyAccesses * b->nrounds;
+  if (get_lock_blob(c, p, dtype, &b)) return 1;     // (the launch reports what is wrong)
+  const size_t esz = (size_t)dtype_size(dtype);
+  return lock_beats_push(b->nrounds, b->saved_rounds, b->accesses, b->bytes, b->nrefs,
+                         (long long)(std::max(p->prog.in_elems, p->prog.out_elems) * (int64_t)esz), (int)esz, lock_on_grid16(c, *b, esz, in, out));
 }
 
 // One launch for a schedule whose tables are on the device (b.dev) or follow from `flat`.
@@ -438,9 +441,7 @@ static int launch_lockstep(chb_comm* c, const chb_comm::LockBlob& b, const FlatS
   int in_smem = flat.coll >= 0 || (b.bytes <= kLockSmemTables && tables_in_smem_wanted()) ? 1 : 0;
   cudaError_t e;
   const size_t tiny_smem = (size_t)b.bytes + (size_t)b.nrefs * sizeof(void*);
-  unsigned long long low = (unsigned long long)b.grid * esz;             // low bits of every address and length
-  for (int l = 0; l < c->P; ++l) low |= (unsigned long long)(uintptr_t)in[l] | (unsigned long long)(uintptr_t)out[l];
-  const bool vec = (low & 15ull) == 0ull;
+  const bool vec = lock_on_grid16(c, b, esz, in, out);
   void* tiny_args[] = {&w, &bp, &bytes, &flat, &io, &op, &scale};
   void* wide_args[] = {&w, &bp, &bytes, &in_smem, &flat, &io, &op, &scale};
   const size_t smem = in_smem ? (size_t)b.bytes : 0;
@@ -452,7 +453,7 @@ static int launch_lockstep(chb_comm* c, const chb_comm::LockBlob& b, const FlatS
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see dependent_launch()
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 1;
-  if (nctas <= 0 && b.accesses <= kTinyAccesses * b.nrounds * (vec ? 16 / (long long)esz : 1) && tiny_smem <= (size_t)kLockSmemTables) {
+  if (nctas <= 0 && lock_one_cta(b.accesses, b.nrounds, b.bytes, b.nrefs, (int)esz, vec)) {
     cfg.gridDim = dim3(1);
     cfg.blockDim = dim3(kTinyThreads);
     cfg.dynamicSmemBytes = tiny_smem;

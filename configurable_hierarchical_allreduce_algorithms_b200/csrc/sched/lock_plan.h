@@ -47,6 +47,7 @@ enum { LOCK_PLAIN = 0, LOCK_COPIES = 1, LOCK_CHAINS = 2 };
 // show), the others accumulate in themselves.
 inline int lock_rewrite_for(int dtype) { return dtype == DT_BF16 || dtype == DT_F16 || dtype == DT_U8 ? LOCK_COPIES : LOCK_CHAINS; }
 LockPlan make_lock_plan(const Program& p, int rewrite);
+inline int lock_saved_rounds(const Program& p, const LockPlan& plan) { return make_lock_plan(p, LOCK_PLAIN).nrounds - plan.nrounds; }
 
 // How a CTA stores the destinations of a step that it has to write (one bit each in `kept`; a copy onto itself is not
 // kept).  mixed: they lie on different 16-byte grids, which the vector loops cannot serve at once; `sources`: those that
@@ -91,6 +92,34 @@ struct LockStep { long long prefix, count, elems; int ref_begin, nsrc, ndst, fin
 struct LockRef { long long off; int rank, buf; };
 static_assert(sizeof(LockHeader) % 16 == 0 && sizeof(LockRound) % 16 == 0 && sizeof(LockStep) % 16 == 0 && sizeof(LockRef) % 16 == 0, "copied as 16-byte words");
 std::vector<char> make_lock_blob(const LockPlan& p);
+inline long long lock_blob_bytes(long long nrounds, long long nsteps, long long nrefs) {
+  return (long long)sizeof(LockHeader) + nrounds * (long long)sizeof(LockRound) + nsteps * (long long)sizeof(LockStep) + nrefs * (long long)sizeof(LockRef);
+}
+
+// May one CTA run the schedule?  accesses: element loads + stores in all; vec: everything on the 16-byte grid.
+constexpr long long kTinyAccesses = 8192;          // loads + stores a round, on average, up to which one CTA runs the schedule
+constexpr long long kLockSmemTables = 40 << 10;    // schedules up to this size are kept in shared memory
+inline bool lock_one_cta(long long accesses, int nrounds, long long bytes, long long nrefs, int esz, bool vec) {
+  return accesses <= kTinyAccesses * nrounds * (vec ? 16 / esz : 1) && bytes + nrefs * (long long)sizeof(void*) <= kLockSmemTables;
+}
+// Does a schedule run faster in lockstep than with flagged lines (kernels/llprog.cu), whose rounds have no barrier but whose
+// data goes through an inbox?  saved: rounds that the rewriting has taken out; payload: bytes of a rank's longer vector.  One
+// round: always, its launch alone is cheaper.  One CTA: a round costs little, but it is one SM.  A cluster or the grid: estimates
+// in halves of a microsecond.  A round costs about 3.5 us more than one of lines and every 10 KB of tables 1.5 us; lines cost
+// 4.5 us where a round is saved and 1 us for each, 0.5 us for each MB that lockstep moves and 20 us for each MB of payload.
+// Made from 6520 schedules timed both ways on one B200 (2 to 16 ranks, 2 B to 4 MiB, all algorithms, any alignment): of those
+// sent here 179 are more than a tenth and 53 more than three tenths slower than with lines, of those sent to lines 31 and 9 slower
+// than in lockstep (with the rounds saved and 192 KiB as the whole rule: 311 and 134, 24 and 9).
+// 16 ranks, in lockstep and with lines: ring reduce-scatter of 1248 bf16 a block 51 and 27 us, recursive doubling of 2.5 KiB fp32
+// 16.5 and 10.4 us, all-to-all of 80 B blocks 25 and 12 us; 8 ranks, allreduce of 256 KiB fp32, k = 4, b = 2, 13.7 and 15.8 us.  The
+// largest misses: a ring reduce-scatter of 16-bit blocks (whose chains are not joined) around 1 MiB, 8 ranks, 44 and 27 us, and
+// hierarchical reduce-scatters of a few hundred bytes a block off the 16-byte grid, 16 ranks, 24 and 12 us.
+inline bool lock_beats_push(int nrounds, int saved, long long accesses, long long bytes, long long nrefs, long long payload, int esz, bool vec) {
+  if (nrounds < 2) return true;
+  if (lock_one_cta(accesses, nrounds, bytes, nrefs, esz, vec)) return (vec ? accesses * esz / 16 : accesses) <= kTinyAccesses / 2 * (3 + 2 * saved + nrounds);
+  if (saved <= 0 && payload <= (192 << 10)) return false;      // (recursive doubling, halving: every round is an exchange that reduces)
+  return 7 * nrounds + 3 * bytes / 10000 <= 13 + (saved > 0 ? 9 + 2 * saved : 0) + ((accesses * esz + 40 * payload) >> 20);
+}
 
 // What the one-shot and two-shot line kernels compute, in these tables: operands in rank order, every rank the same result.
 // One round: an allreduce is one step (all inputs, all outputs), a reduce-scatter and an allgather one step per block.  It

@@ -223,6 +223,11 @@ class Program:
             raise RuntimeError(f"lock_info failed with code {rc}")
         return dict(zip(("rounds", "steps", "reads", "stores"), [int(x) for x in v]))
 
+    def lock_preferred(self, dtype: int, on_grid16: bool = True) -> bool:
+        """Whether an emulated world runs this program in lockstep where flagged lines could carry it too (``dtype``: the
+        native code, ``parallel.comm.DTYPES``)."""
+        return bool(N.lib().chb_program_lock_preferred(self._h, int(dtype), int(on_grid16)))
+
     def simulate_ll(self, inputs: list[np.ndarray], op: str = "sum", seed: int = 0, threads: int = 5,
                     fault: int = 0, launches: int = 1) -> list[np.ndarray]:
         """Run the push (flagged-line) form of this program on host arrays, line by line, the way the GPU executor

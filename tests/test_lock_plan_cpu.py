@@ -96,3 +96,18 @@ def test_flat_schedule_without_a_program(P):
             blocks = [x[:n].copy() for x in xs]
             for got in chb.Program.simulate_flat("allgather", blocks, seed=seed):
                 assert got.tobytes() == np.concatenate(blocks).tobytes()
+
+
+@pytest.mark.parametrize("coll,algo,P,k,b,block,dtype,grid16,lockstep", [
+    # many rounds that the rewriting keeps: faster with flagged lines (16 ranks unless said otherwise)
+    ("reduce_scatter", "ring", 16, 2, 1, 1248, 1, True, False), ("reduce_scatter", "pairwise", 16, 2, 1, 1248, 1, False, False),
+    ("allreduce", "recursive_doubling", 16, 2, 1, 40, 0, True, False), ("allreduce", "recursive_doubling", 16, 2, 1, 40, 0, False, False),
+    ("reduce_scatter", "recursive_halving", 16, 2, 1, 160, 1, False, False), ("alltoall", "tuna", 16, 2, 1, 40, 1, True, False),
+    # one round, few rounds, or much data: faster in lockstep
+    ("allreduce", "radix_batch", 8, 2, 1, 1248, 0, False, True), ("allreduce", "ring", 8, 2, 1, 4096, 0, True, True),
+    ("allreduce", "radix_batch", 8, 4, 2, 131072, 0, True, True), ("allreduce", "radix_batch", 8, 8, 8, 1, 0, True, True),
+    ("allreduce", "radix_batch", 8, 2, 4, 128, 0, True, True), ("alltoall", "linear", 8, 2, 1, 160, 0, True, True),
+    ("reduce_scatter", "radix_batch", 8, 4, 2, 1248, 1, True, True)])
+def test_lockstep_where_it_is_faster_than_flagged_lines(coll, algo, P, k, b, block, dtype, grid16, lockstep):
+    p = chb.Program(coll, algo, P, block * P if coll == "allreduce" else block, k, b, in_symmetric=True, out_symmetric=True)
+    assert p.lock_preferred(dtype, grid16) == lockstep
