@@ -1,9 +1,11 @@
 """Kernels on a real GPU with all ranks emulated on that one device.
 
 Each kernel is compared against a plain PyTorch fp32 / fp64 reference of the
-same collective.  The emulated world runs the same kernels as a multi-GPU
-world: the peers' heaps are slices of one allocation and one cooperative
-launch executes all ranks.
+same collective.  The peers' heaps are slices of one allocation and one launch
+executes all ranks: schedules without an execution-mode suffix in lockstep,
+the bulk allgather in its local form, and with ``:pull`` and ``:ll`` the
+kernels of a multi-GPU world (``test_gpu_per_rank_kernels.py`` makes the same
+calls on those).
 """
 import pytest
 import torch
@@ -338,7 +340,8 @@ def test_in_place_flagged_line_kernels(comms):
 
 @pytest.mark.parametrize("P", [2, 4, 8])
 def test_bulk_copy_allgather(comms, P):
-    """Allgather through the bulk-copy engine (shared-memory ring, mbarriers)."""
+    """Allgather under the name of the bulk-copy engine: with all ranks on one GPU the form that reads every block once,
+    in a traced world the ring through shared memory."""
     comm = comms(P)
     for dtype, n in ((torch.float32, 4), (torch.float32, 2052), (torch.bfloat16, 8 * 3001), (torch.float32, (1 << 20) + 12)):
         xs = comm.empty(n, dtype)
