@@ -15,6 +15,7 @@
 
 #include "sched/algos.h"
 #include "sched/ll_plan.h"
+#include "sched/lock_plan.h"
 #include "sched/program.h"
 #include "sched/types.h"
 
@@ -125,10 +126,79 @@ void run_case(const AlgoSpec& s, bool threads_only) {
       if (simulate_ll(p, DT_I32, OP_SUM, ip.data(), op.data(), 17u, 3, LL_FAULT_NONE, 2, &err) != 0) fail("simulate_ll", s, err);
       else check("simulate_ll");
     }
+    // the lockstep form: rewriting, tables, and execution with the steps of a round in random order
+    if (!threads_only)
+      for (int rewrite = LOCK_PLAIN; rewrite <= LOCK_CHAINS; ++rewrite) {
+        for (auto& v : out) std::fill(v.begin(), v.end(), -1);
+        if (make_lock_blob(make_lock_plan(p, rewrite)).empty()) fail("make_lock_blob", s, "no tables");
+        if (simulate_lock(p, DT_I32, OP_SUM, ip.data(), op.data(), 23u + rewrite, rewrite, &err) != 0) fail("simulate_lock", s, err);
+        else check("simulate_lock");
+      }
     for (auto& v : out) std::fill(v.begin(), v.end(), -1);
     double sec = 0;
     if (run_threads(p, DT_I32, OP_SUM, ip.data(), op.data(), 2, &sec) != 0) fail("run_threads", s, "wait expired");
     else check("run_threads");
+  }
+}
+
+// An allreduce in place on buffers that lie on different 16-byte grids, in lockstep: steps that store to several of their
+// own operands.
+void run_in_place(const AlgoSpec& s) {
+  Builder B(1, 0, 0, "");
+  try {
+    B = build_algorithm(s);
+  } catch (const std::runtime_error&) {
+    return;
+  }
+  LowerOpts o;
+  o.in_place = true;
+  Program p = B.lower(o);
+  ++g_cases;
+  for (int rewrite = LOCK_PLAIN; rewrite <= LOCK_CHAINS; ++rewrite) {
+    std::vector<std::vector<int32_t>> buf(s.P);
+    std::vector<void*> at(s.P);
+    for (int r = 0; r < s.P; ++r) {
+      buf[r].assign(p.out_elems + r % 4, -1);
+      at[r] = buf[r].data() + r % 4;
+      for (int64_t i = 0; i < p.in_elems; ++i) buf[r][r % 4 + i] = value(r, i);
+    }
+    std::string err;
+    if (simulate_lock(p, DT_I32, OP_SUM, at.data(), at.data(), 5u + rewrite, rewrite, &err) != 0) { fail("in place", s, err); continue; }
+    std::vector<int32_t> e;
+    for (int r = 0; r < s.P; ++r) {
+      int me = 0;
+      const std::vector<int> members = members_of(s, r, &me);
+      if (!expect(s.coll, members, me, p.in_elems, p.out_elems, 0, e)) continue;
+      if (std::memcmp(e.data(), at[r], sizeof(int32_t) * p.out_elems) != 0) { fail("in place", s, "wrong result on rank " + std::to_string(r)); break; }
+    }
+  }
+}
+
+// The flat schedule, which a CTA writes itself.
+void run_flat(int coll, int P, int64_t n) {
+  ++g_cases;
+  std::vector<std::vector<int32_t>> in(P), out(P);
+  std::vector<void*> ip(P), op(P);
+  for (int r = 0; r < P; ++r) {
+    in[r].resize(coll == 1 ? n * P : n);
+    out[r].assign(coll == 2 ? n * P : n, -1);
+    for (size_t i = 0; i < in[r].size(); ++i) in[r][i] = value(r, (int64_t)i);
+    ip[r] = in[r].data();
+    op[r] = out[r].data();
+  }
+  std::string err;
+  AlgoSpec s;
+  s.coll = coll == 0 ? "allreduce" : coll == 1 ? "reduce_scatter" : "allgather";
+  s.algo = "flat";
+  s.P = P;
+  s.count = n;
+  if (simulate_flat(FlatSpec{coll, 0, n}, P, DT_I32, OP_SUM, ip.data(), op.data(), (uint64_t)n, &err) != 0) { fail("flat", s, err); return; }
+  std::vector<int> members(P);
+  for (int r = 0; r < P; ++r) members[r] = r;
+  std::vector<int32_t> e;
+  for (int r = 0; r < P; ++r) {
+    expect(s.coll, members, r, (int64_t)in[r].size(), (int64_t)out[r].size(), 0, e);
+    if (e != out[r]) { fail("flat", s, "wrong result on rank " + std::to_string(r)); return; }
   }
 }
 
@@ -164,11 +234,16 @@ int main(int argc, char** argv) {
             // allreduce counts are totals (a multiple of P), the others are per block; 5 keeps ragged tails in play
             s.count = std::string(coll) == "allreduce" ? (int64_t)P * 5 : 5;
             run_case(s, threads_only);
+            if (!threads_only && std::string(coll) == "allreduce") run_in_place(s);
           }
         }
       }
     }
   }
+  if (!threads_only)
+    for (int coll = 0; coll < 3; ++coll)
+      for (int P : {2, 3, 8, 16})
+        for (int64_t n : {1, 5, 2049}) run_flat(coll, P, n);
   std::printf("%d programs, %d failures\n", g_cases, g_fail);
   return g_fail ? 1 : 0;
 }
