@@ -510,7 +510,7 @@ static int get_blob(chb_comm* c, const chb_program* p, void** out) {
   std::vector<char> blob = make_blob(p->prog, &table_bytes);
   void* d = nullptr;
   if (cudaMalloc(&d, blob.size()) != cudaSuccess) { c->last_error = "cudaMalloc(program blob) failed"; return CHB_ERR_NO_MEM; }
-  if (cudaMemcpy(d, blob.data(), blob.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (upload_table(d, blob) != cudaSuccess) {
     cudaFree(d);
     c->last_error = "cudaMemcpy(program blob) failed";
     return CHB_ERR_CUDA;

@@ -365,7 +365,7 @@ int chb_run_program_ll(chb_comm* c, const chb_program* p, int dtype, int op, con
       return CHB_ERR_COUNT;
     }
     if (cudaMalloc(&blob, host.size()) != cudaSuccess) { c->last_error = "cudaMalloc(program lines) failed"; return CHB_ERR_NO_MEM; }
-    if (cudaMemcpy(blob, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload_table(blob, host) != cudaSuccess) {
       cudaFree(blob);
       c->last_error = "cudaMemcpy(program lines) failed";
       return CHB_ERR_CUDA;

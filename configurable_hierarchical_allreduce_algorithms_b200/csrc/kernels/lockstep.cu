@@ -389,7 +389,7 @@ static int get_lock_blob(chb_comm* c, const chb_program* p, int dtype, const chb
     const std::vector<char> host = make_lock_blob(plan);
     b.bytes = (int)host.size();
     if (cudaMalloc(&b.dev, host.size()) != cudaSuccess) { c->last_error = "cudaMalloc(lockstep schedule) failed"; return CHB_ERR_NO_MEM; }
-    if (cudaMemcpy(b.dev, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload_table(b.dev, host) != cudaSuccess) {
       cudaFree(b.dev);
       c->last_error = "cudaMemcpy(lockstep schedule) failed";
       return CHB_ERR_CUDA;

@@ -73,6 +73,13 @@ struct Program;
 bool program_ranges_ok(const Program& p, std::string* why);
 }
 
+// Copies a schedule's tables to the device and waits until they are there: a copy from pageable memory may return while its
+// last part is still on the way, and a launch on a non-blocking stream would not wait for it.
+inline cudaError_t upload_table(void* dev, const std::vector<char>& host) {
+  const cudaError_t e = cudaMemcpyAsync(dev, host.data(), host.size(), cudaMemcpyHostToDevice, cudaStreamLegacy);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // CHB_TABLES_IN_SMEM=0 keeps the program kernels' schedule tables in global memory (for A/B timing and debugging)
 inline bool tables_in_smem_wanted() {
   static const bool on = [] {

@@ -30,3 +30,13 @@ def test_no_read_only_promise_in_overlapped_kernels():
                 assert pointer in NEVER_WRITTEN, f"{f.name}: {name}({pointer})"
         seen += len(overlapped)
     assert seen >= 8
+
+
+def test_tables_have_arrived_before_a_launch_reads_them():
+    """A blocking copy from pageable memory may return before its last part is on the device, and launches on non-blocking
+    streams do not wait for it: uploads that kernels read go through the helper that waits."""
+    for f in sorted(KERNELS.parent.rglob("*.cu")):
+        if "tools" not in f.parts:
+            assert not re.search(r"\bcudaMemcpy\([^;]*HostToDevice", f.read_text()), f.name
+    helper = next(body for name, _, body in functions((KERNELS.parent / "symm" / "comm.h").read_text()) if name == "upload_table")
+    assert helper.index("cudaMemcpyHostToDevice") < helper.index("cudaStreamSynchronize")
