@@ -238,8 +238,8 @@ int chb_collective(chb_comm* c, int coll, const char* algo, int k, int b, int au
 // A call that the flagged-line kernels `ll` (two_shot = 0) or `ll2` (two_shot = 1) would take, with all ranks on this GPU: the
 // same result, bit for bit, in lockstep.  ptrs: the ranks' inputs, then their outputs.  CHB_ERR_UNSUPPORTED, and nothing
 // launched, where the line kernels have to run (one rank per GPU, traced, overlapping buffers) or would refuse.
-// 8 ranks, fp32 allreduce of 32 KiB / 256 KiB / 1 MiB: 7.5 / 18 / 72 us one-shot, 12 / 12.8 / 21.6 us two-shot, 7.4 / 9.2 /
-// 9.6 us in lockstep.
+// 8 ranks, fp32 allreduce of 32 KiB / 256 KiB / 1 MiB in a graph: 7.4 / 18.1 / 21.8 us with the line kernel that the tuned table
+// names, 8.8 / 9.2 / 9.3 us in lockstep; called one by one 32 KiB take 15.8 and 9.3 us (the host's part).
 int chb_collective_local(chb_comm* c, int coll, int two_shot, int dtype, int op, const char* ptrs, int64_t count, float scale,
                          cudaStream_t stream) {
   if (!c || !ptrs || count <= 0 || c->nlocal != c->P || c->P < 2 || coll < CHB_ALLREDUCE || coll > CHB_ALLGATHER) return CHB_ERR_UNSUPPORTED;

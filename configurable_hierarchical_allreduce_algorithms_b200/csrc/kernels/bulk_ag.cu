@@ -168,8 +168,8 @@ ag_bulk_kernel(World w, BulkIo io, long long nbytes) {
 // nobody else writes).
 // Bound by HBM writes: P - 1 of P bytes moved are stores.  Plain vector stores from many short CTAs, four vectors a thread
 // (one piece of 32 KiB a CTA, all CTAs in one moving window of every output); a ring of bulk copies, one stage stored P
-// times by one thread an SM, ran at 115 us where this takes 94.
-// Measured on one B200, 8 ranks, 8 MiB of bf16 a rank: 166 us fetching P times -> 94 us (604 MB in and out: 6.4 TB/s).
+// times by one thread an SM, ran at 115 us where this takes 92.
+// Measured on one B200, 8 ranks, 8 MiB of bf16 a rank: 166 us fetching P times -> 92.5 us (604 MB in and out: 6.5 TB/s).
 constexpr int kLocalThreads = 256, kLocalUnroll = 4;
 
 // WIDE: 32-byte vectors (every pointer and the block length a multiple of 32), else 16-byte ones.

@@ -109,7 +109,7 @@ rs_adam_kernel(World w, AdamIo io, long long n, AdamHyper h, const char* mc_grad
 // anybody, and the shards need no persistent CTAs that meet at barriers.
 // Bound by HBM: 4 P + 26 bytes an element of a shard.  One vector of four elements a thread, all P gradient loads (in
 // batches of eight) and the three state loads issued before the first addition, short CTAs.
-// Measured on one B200, 8 ranks x 2 Mi elements a shard: 235 us with barriers and 18 CTAs a rank, 199 us so (each with the allgather
+// Measured on one B200, 8 ranks x 2 Mi elements a shard: 235 us with barriers and 18 CTAs a rank, 190 us so (each with the allgather
 // of the parameters, 1.2 GB in all).
 constexpr int kLocalAdamThreads = 256;
 

@@ -280,7 +280,7 @@ __device__ __noinline__ RankTables tables_to_smem(const char* __restrict__ blob,
 }
 
 // Where a CTA is in the schedule.  In shared memory rather than in registers: nothing of it is then live across the
-// call that runs a span (see run_span).
+// loops that run a span (see run_span, which is inlined).
 struct RoundWalk {
   const DevRound* rounds;
   const DevStep* steps;

@@ -16,7 +16,7 @@
 // cooperative launch unless there is one round only (3.5 us a round, 148 CTAs).
 // Measured on one B200 with 8 emulated ranks, per-rank kernels -> this: allreduce 4 MiB fp32 k = 4, b = 2 113 -> 30 us
 // (67 MB in and out: 2.2 TB/s), 25 MiB fp32 143 (101 with the loops of span.cuh) -> 84 us (419 MB: 5.0 TB/s),
-// reduce-scatter of 8 x 1,000,003 bf16 1238 (144) -> 77 us, k = 2, b = 4 of 4 KiB 12.5 -> 6.8 us.
+// reduce-scatter of 8 x 1,000,003 bf16 1238 (144) -> 66 us, k = 2, b = 4 of 4 KiB 12.5 -> 6.8 us.
 //
 // The ranks' epochs and signal pads are left alone (nobody is signalled and nobody waits), so launches of this kernel
 // and of the per-rank ones mix freely on one communicator.

@@ -35,7 +35,8 @@ __device__ __forceinline__ void vec_combine_as(int op, const uint4& v, typename 
 }
 
 // 256-bit loop over vectors [j0, nw) strided by TT: G sources x UW vectors in flight per thread.
-// (not inlined: each variant gets a register allocation of its own instead of inflating its caller's)
+// (all loops here are inlined into their kernel; the callers keep their span and their place in the schedule in shared
+// memory, so that little else competes for registers)
 template <typename T, bool SUM, int G, int UW>
 __device__ __forceinline__ void reduce_loop32(const char* const* src, long long sofs, int nsrc, char* const* dst, int ndst, long long dofs,
                                            int j0, int nw, int TT, int op, bool do_scale, float scale) {

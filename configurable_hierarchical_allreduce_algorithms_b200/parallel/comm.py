@@ -5,7 +5,8 @@ Two flavours share every code path below the constructor:
 * ``Communicator.emulated(P)`` — all P ranks live on ONE GPU (P slices of one
   allocation, one launch executes every rank).  Used by the single-GPU tests and
   for developing schedules without a multi-GPU box.  Step programs run in lockstep
-  there unless their name pins ``:pull`` or ``:ll``, the kernels of separate GPUs.
+  there (small ones of many rounds with flagged lines, where those are expected to
+  be faster) unless their name pins ``:pull`` or ``:ll``, the kernels of separate GPUs.
 * ``Communicator.from_process_group(group)`` — one rank per process / GPU over
   NVLink; heaps are exchanged either as cudaIpc handles (``backend="ipc"``,
   native) or through ``torch.distributed._symmetric_memory``
