@@ -28,7 +28,8 @@ int chb_lockstep_ok(const chb_comm* c, const chb_program* p, int dtype, const vo
 int chb_run_flat_lockstep(chb_comm* c, int coll, int dtype, int op, const void* const* in, void* const* out, long long n,
                           float scale, cudaStream_t stream);
 int chb_program_fits(const chb_comm* c, const chb_program* p, int dtype);
-int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out);
+int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, const void* const* in, void* const* out,
+                            cudaStream_t stream);
 long long chb_program_ll_lines(const chb_program* p, int esz);
 int chb_ll_collective(chb_comm* c, int mode, int dtype, int op, const void* const* in, void* const* out,
                       long long count, float scale, int nctas, cudaStream_t stream);
@@ -215,7 +216,7 @@ int chb_collective(chb_comm* c, int coll, const char* algo, int k, int b, int au
       if (rc) return rc;
       const long long need = chb_program_ll_lines(p, esz);
       if (mode == 0 && need <= (long long)c->P * (long long)c->ll_lines_per_src && chb_lockstep_ok(c, p, dtype, in, out, slot) &&
-          chb_lockstep_beats_push(c, p, dtype, in, out))
+          chb_lockstep_beats_push(c, p, dtype, in, out, stream))
         return chb_run_program_lockstep(c, p, dtype, op, in, out, scale, nctas, stream);
       if (need <= (long long)c->P * (long long)c->ll_lines_per_src)
         return chb_run_program_ll(c, p, dtype, op, in, out, scale, nctas, stream);

@@ -252,3 +252,24 @@ def test_first_call_of_a_length_may_be_captured(cuda):
         assert torch.equal(ag[r], torch.cat(blocks))
     comm.check()
     comm.close()
+
+
+def test_a_captured_call_keeps_to_tables_that_are_there(cuda):
+    """Recursive doubling of 512 elements runs in lockstep on aligned buffers and with flagged lines on skewed ones: captured
+    on skewed buffers after calls on aligned ones it stays in lockstep, where no table has to be uploaded."""
+    P, n = 8, 512
+    p = chb.Program("allreduce", "recursive_doubling", P, n, 2, 1, in_symmetric=True, out_symmetric=True)
+    assert p.lock_preferred(0, True) and not p.lock_preferred(0, False)
+    comm = Communicator.emulated(P, scratch_bytes=4 << 20, user_bytes=4096)
+    src = [torch.randn(n + 1, device="cuda") for _ in range(P)]
+    chb.all_reduce(comm, [s[:n].clone() for s in src], algo="recursive_doubling")
+    chb.all_reduce(comm, [s[1:3] for s in src], algo="recursive_doubling")      # (loads the kernel for other alignments)
+    ins, outs = [s[1:] for s in src], [torch.zeros(n + 1, device="cuda")[1:] for _ in range(P)]
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        chb.all_reduce(comm, ins, out=outs, algo="recursive_doubling")
+    graph.replay()
+    want = chb.all_reduce(comm, ins, algo="recursive_doubling:pull")
+    assert all(torch.equal(x, y) for x, y in zip(outs, want))
+    comm.check()
+    comm.close()
