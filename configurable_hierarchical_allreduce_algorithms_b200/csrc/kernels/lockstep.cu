@@ -415,12 +415,13 @@ int chb_lockstep_beats_push(chb_comm* c, const chb_program* p, int dtype, const 
   const chb_comm::LockBlob* b = nullptr;
   if (get_lock_blob(c, p, dtype, &b)) return 1;     // (the launch reports what is wrong)
   const size_t esz = (size_t)dtype_size(dtype);
+  if (lock_beats_push(b->nrounds, b->saved_rounds, b->accesses, b->bytes, b->nrefs,
+                      (long long)(std::max(p->prog.in_elems, p->prog.out_elems) * (int64_t)esz), (int)esz, lock_on_grid16(c, *b, esz, in, out)))
+    return 1;
   // A captured call cannot upload the tables of the lines: one whose alignment would send it there, unlike that of the calls
   // before it, stays in lockstep, whose tables are up.
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (!c->ll_blobs.count(p->uid * 16u + esz) && cudaStreamIsCapturing(stream, &capturing) == cudaSuccess && capturing != cudaStreamCaptureStatusNone) return 1;
-  return lock_beats_push(b->nrounds, b->saved_rounds, b->accesses, b->bytes, b->nrefs,
-                         (long long)(std::max(p->prog.in_elems, p->prog.out_elems) * (int64_t)esz), (int)esz, lock_on_grid16(c, *b, esz, in, out));
+  return !c->ll_blobs.count(p->uid * 16u + esz) && cudaStreamIsCapturing(stream, &capturing) == cudaSuccess && capturing != cudaStreamCaptureStatusNone;
 }
 
 // One launch for a schedule whose tables are on the device (b.dev) or follow from `flat`.
